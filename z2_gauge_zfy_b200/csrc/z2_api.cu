@@ -42,7 +42,6 @@ __device__ __forceinline__ void load_desc(ChainDesc &sc, const ChainDesc *g) {
 __global__ void __launch_bounds__(Z2_NT, 1)
 z2_chain_kernel(const ChainDesc *descs, const int *order, int nchains, int *queue, int op,
                 int nsweep, int toggle, unsigned smem_bytes) {
-  extern __shared__ __align__(16) unsigned char z2_smem[];
   __shared__ ChainDesc sc;
   __shared__ Smem s;     // pointer table in shared memory, not on the local stack
   __shared__ int s_idx;
@@ -77,7 +76,6 @@ z2_state_kernel(const ChainDesc *desc, int op, int nt, int flag, double x, unsig
 // Module-level mirrors on single matrices, one CTA.
 __global__ void __launch_bounds__(Z2_NT, 1)
 z2_unit_kernel(const ChainDesc *desc, int op, UnitArgs a, unsigned smem_bytes) {
-  extern __shared__ __align__(16) unsigned char z2_smem[];
   __shared__ ChainDesc sc;
   __shared__ Smem s;
   load_desc(sc, desc);
@@ -341,12 +339,12 @@ static size_t tile_min(int N) {
   return t;
 }
 
-static int default_k(int N) {
-  if (N <= 36) return 16;
-  if (N <= 64) return 16;
-  if (N <= 100) return 12;
-  return 8;
-}
+// Delayed-update rank when the caller names none: the columns of an accept
+// cost a loop over the queued pairs, a flush its fragment loads.  Cycles per
+// accept of a slice at ranks 4 / 8 / 16: 1764 / 1701 / 1761 (N = 64), and
+// 3.8 K / 3.1 K / 3.0 K at ranks 2 / 4 / 8 (N = 144, where 8 fills shared
+// memory); flat below N = 64.
+static const int kDefaultRank = 8;
 
 extern "C" int z2_create(z2_handle **out, const z2_chain_params *params, int32_t nchains,
                          const z2_options *opt) {
@@ -410,7 +408,7 @@ extern "C" int z2_create(z2_handle **out, const z2_chain_params *params, int32_t
     // otherwise (conflict-free strided rows)
     const int ldg = (N % 4 == 0) ? N + 2 : ((N % 2) ? N : N + 1);
     int small = smem_small_bytes(N);
-    int k = h->opt.delay_k > 0 ? h->opt.delay_k : default_k(N);
+    int k = h->opt.delay_k > 0 ? h->opt.delay_k : kDefaultRank;
     if (h->opt.delay_k_chain && h->opt.delay_k_chain[c] > 0) k = h->opt.delay_k_chain[c];
     if (k > 64) k = 64;
     size_t arena = (size_t)(kSmemMax - small) / 8;
@@ -1026,8 +1024,9 @@ static int probe_cycles(const std::vector<z2_chain_params> &probe, const z2_opti
 // lattice size: three probe chains per size (the chain's couplings and time
 // step, Ltrot cut to 2 Nwrap), every size side by side in one launch per
 // candidate, the median SM cycles of the three, and the first candidate in
-// preference order (default shape, then smaller rank) within 3 % of the
-// fastest.
+// preference order (default shape and rank, then default shape and smaller
+// ranks) within 5 % of the fastest: the ranks' times lie within a few percent
+// of each other, and run-to-run noise in the probes must not flip the pick.
 static int tune_core(const z2_chain_params *params, int nchains, const z2_options *opt,
                      bool shapes, int32_t *k_out, int32_t *shape_out) {
   if (!params || nchains <= 0 || !k_out) return Z2_ERR_ARG;
@@ -1059,7 +1058,11 @@ static int tune_core(const z2_chain_params *params, int nchains, const z2_option
   base.stab_exact = opt ? opt->stab_exact : 0;
   // the ranks shared memory allows for each size (no launch: the plan only)
   std::vector<std::vector<int>> ks(ns);
-  for (int k : kTuneCand) {
+  // the default rank first: it is kept unless another is clearly faster
+  std::vector<int> ranks{kDefaultRank};
+  for (int k : kTuneCand)
+    if (k != kDefaultRank) ranks.push_back(k);
+  for (int k : ranks) {
     z2_options o = base;
     o.delay_k = k;
     z2_handle *h = nullptr;
@@ -1107,7 +1110,7 @@ static int tune_core(const z2_chain_params *params, int nchains, const z2_option
   for (int i = 0; i < ns; ++i) {
     const double best = *std::min_element(cost[i].begin(), cost[i].end());
     for (size_t ci = 0; ci < cands[i].size(); ++ci)
-      if (cost[i][ci] <= 1.03 * best) { pick[i] = cands[i][ci]; break; }
+      if (cost[i][ci] <= 1.05 * best) { pick[i] = cands[i][ci]; break; }
   }
   for (int c = 0; c < nchains; ++c) {
     const int N = params[c].Nlx * params[c].Nly;
@@ -1356,7 +1359,6 @@ enum {
 
 __global__ void __launch_bounds__(Z2_NT, 1)
 z2_state_kernel(const ChainDesc *desc, int op, int nt, int flag, double x, unsigned smem_bytes) {
-  extern __shared__ __align__(16) unsigned char z2_smem[];
   __shared__ ChainDesc sc;
   __shared__ Smem s;
   load_desc(sc, desc);
@@ -1666,7 +1668,6 @@ __global__ void __launch_bounds__(Z2_NT, 1)
 z2_stab_green_noalloc_kernel(int N, int nt, int Ltrot, const double *UR, const double *DR,
                              const double *VR, const double *UL, const double *DL,
                              const double *VL, double *G, double *scratch) {
-  extern __shared__ __align__(16) unsigned char z2_smem[];
   Smem s{};
   size_t off = 0;
   s.red = (double *)(z2_smem + off); off += sizeof(double) * Z2_NRED;

@@ -9,6 +9,7 @@
 // update, and the U factors of the UDV chains are propagated lazily (all
 // Nwrap slices at once, right before the stabilization that needs them).
 #pragma once
+#include "z2_propose.cuh"
 #include "z2_stab.cuh"
 
 // Checkerboard group order of one B (src/operator_kin.f90:74-85).
@@ -521,358 +522,6 @@ __device__ __noinline__ void green_big_extract(int N, const double *B3, double *
 }
 
 // ---------------------------------------------------------------------------
-// Delayed rank-2 updates (LocalK_metro, src/localK.f90:45-173)
-// ---------------------------------------------------------------------------
-// The delayed-update factors X and Yt (N x k2 each) keep their columns in
-// interleaved pairs: element (i, q) sits at (q / 2) 2 ldx + 2 i + q % 2, so
-// the two columns an accepted flip adds are one 16-byte word per row (one
-// load in the ratio evaluation and in the column phase, one store), and a
-// DMMA fragment (rows r + 0..7, columns l + 0..3) still hits 16 distinct
-// bank pairs per half-warp for ldx = 4 (mod 16).
-__device__ __forceinline__ size_t xy_at(int i, int q, int ldx) {
-  return (size_t)(q >> 1) * (2 * ldx) + 2 * i + (q & 1);
-}
-
-// G <- G - X Yt^T over the m queued columns (paired layout) when 8 TR and 8 TC
-// divide N: each warp owns (8 TR) x (8 TC) blocks of G, loads their old
-// values straight into the DMMA accumulators and adds (-X) Yt^T to them in
-// chunks of 4 columns, reusing each X fragment TC times and each Yt fragment
-// TR times.
-template <int TR, int TC>
-__device__ __noinline__ void flush_tiles(double *G, int ldg, const double *X, const double *Yt,
-                                         int N, int ldx, int m) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int lr = lane >> 2, lc = lane & 3;
-  const int gr = N / (8 * TR), gcn = N / (8 * TC);
-  const int m4 = m & ~3;
-  const size_t s4 = (size_t)4 * ldx;
-  for (int g = warp; g < gr * gcn; g += Z2_WARPS) {
-    const int r0 = (g % gr) * 8 * TR, c0 = (g / gr) * 8 * TC;
-    double *cp = G + r0 + lr + (size_t)(c0 + 2 * lc) * ldg;
-    double acc[TR][TC][2];
-#pragma unroll
-    for (int a = 0; a < TR; ++a)
-#pragma unroll
-      for (int b = 0; b < TC; ++b)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) acc[a][b][e] = cp[8 * a + (size_t)(8 * b + e) * ldg];
-    const double *pa = X + xy_at(r0 + lr, lc, ldx);
-    const double *pb = Yt + xy_at(c0 + lr, lc, ldx);
-#pragma unroll 2
-    for (int l0 = 0; l0 < m4; l0 += 4) {
-      double fa[TR], fb[TC];
-#pragma unroll
-      for (int u = 0; u < TR; ++u) fa[u] = -pa[16 * u];
-#pragma unroll
-      for (int v = 0; v < TC; ++v) fb[v] = pb[16 * v];
-      pa += s4; pb += s4;
-#pragma unroll
-      for (int u = 0; u < TR; ++u)
-#pragma unroll
-        for (int v = 0; v < TC; ++v) dmma884(acc[u][v][0], acc[u][v][1], fa[u], fb[v]);
-    }
-    if (m4 < m) {
-      // two trailing columns: lanes lc >= m - m4 feed zeros
-      const bool ok = lc < m - m4;
-      double fa[TR], fb[TC];
-#pragma unroll
-      for (int u = 0; u < TR; ++u) fa[u] = ok ? -pa[16 * u] : 0.0;
-#pragma unroll
-      for (int v = 0; v < TC; ++v) fb[v] = ok ? pb[16 * v] : 0.0;
-#pragma unroll
-      for (int u = 0; u < TR; ++u)
-#pragma unroll
-        for (int v = 0; v < TC; ++v) dmma884(acc[u][v][0], acc[u][v][1], fa[u], fb[v]);
-    }
-#pragma unroll
-    for (int a = 0; a < TR; ++a)
-#pragma unroll
-      for (int b = 0; b < TC; ++b)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) cp[8 * a + (size_t)(8 * b + e) * ldg] = acc[a][b][e];
-  }
-  __syncthreads();
-}
-
-// The same update for any N: (8 GS) x (8 GS) groups with bounds checks.
-template <int GS>
-__device__ __noinline__ void flush_generic(double *G, int ldg, const double *X, const double *Yt,
-                                           int N, int ldx, int m) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int lr = lane >> 2, lc = lane & 3;
-  const int gm = (N + 8 * GS - 1) / (8 * GS);
-  for (int g = warp; g < gm * gm; g += Z2_WARPS) {
-    const int r0 = (g % gm) * 8 * GS, c0 = (g / gm) * 8 * GS;
-    double acc[GS][GS][2];
-#pragma unroll
-    for (int a = 0; a < GS; ++a)
-#pragma unroll
-      for (int b = 0; b < GS; ++b)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int row = r0 + 8 * a + lr, col = c0 + 8 * b + 2 * lc + e;
-          acc[a][b][e] = (row < N && col < N) ? G[row + (size_t)col * ldg] : 0.0;
-        }
-    for (int l0 = 0; l0 < m; l0 += 4) {
-      const int l = l0 + lc;
-      const bool lk = l < m;
-      double fa[GS], fb[GS];
-#pragma unroll
-      for (int u = 0; u < GS; ++u) {
-        const int ra = r0 + 8 * u + lr, cb = c0 + 8 * u + lr;
-        fa[u] = (lk && ra < N) ? -X[xy_at(ra, l, ldx)] : 0.0;
-        fb[u] = (lk && cb < N) ? Yt[xy_at(cb, l, ldx)] : 0.0;
-      }
-#pragma unroll
-      for (int u = 0; u < GS; ++u)
-#pragma unroll
-        for (int v = 0; v < GS; ++v) dmma884(acc[u][v][0], acc[u][v][1], fa[u], fb[v]);
-    }
-#pragma unroll
-    for (int a = 0; a < GS; ++a)
-#pragma unroll
-      for (int b = 0; b < GS; ++b)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int row = r0 + 8 * a + lr, col = c0 + 8 * b + 2 * lc + e;
-          if (row < N && col < N) G[row + (size_t)col * ldg] = acc[a][b][e];
-        }
-  }
-  __syncthreads();
-}
-
-// Tile shapes of the rank-2k flush (z2_options.flush_shape_chain).  Every
-// shape forms each element of G from its old value with the same k chunks,
-// so they give the same bits; they differ in how the N x N update
-// is cut into warp blocks (load balance over the 8 warps against fragment
-// reuse).  0 picks by divisibility: 24 x 24 blocks when 24 | N, 16 x 16 when
-// 16 | N, else the bounded 16 x 16 groups.
-enum {
-  FS_DEFAULT = 0, FS_GEN16 = 1, FS_GEN8 = 2, FS_T11 = 3, FS_T22 = 4, FS_T33 = 5, FS_T21 = 6,
-  FS_T32 = 7, FS_COUNT = 8
-};
-__host__ __device__ __forceinline__ bool flush_shape_ok(int shape, int N) {
-  switch (shape) {
-    case FS_DEFAULT: case FS_GEN16: case FS_GEN8: return true;
-    case FS_T11: return N % 8 == 0;
-    case FS_T22: case FS_T21: return N % 16 == 0;
-    case FS_T33: return N % 24 == 0;
-    case FS_T32: return N % 48 == 0;
-    default: return false;
-  }
-}
-
-// G <- G - X Yt^T over the m queued columns: one DMMA rank-m update.
-__device__ __forceinline__ void rank_update(double *G, int ldg, const double *X, const double *Yt,
-                                            int N, int ldx, int m, int shape = FS_DEFAULT) {
-  switch (shape) {
-    case FS_GEN16: flush_generic<2>(G, ldg, X, Yt, N, ldx, m); return;
-    case FS_GEN8: flush_generic<1>(G, ldg, X, Yt, N, ldx, m); return;
-    case FS_T11: flush_tiles<1, 1>(G, ldg, X, Yt, N, ldx, m); return;
-    case FS_T22: flush_tiles<2, 2>(G, ldg, X, Yt, N, ldx, m); return;
-    case FS_T33: flush_tiles<3, 3>(G, ldg, X, Yt, N, ldx, m); return;
-    case FS_T21: flush_tiles<2, 1>(G, ldg, X, Yt, N, ldx, m); return;
-    case FS_T32: flush_tiles<3, 2>(G, ldg, X, Yt, N, ldx, m); return;
-    default: break;
-  }
-  if (N % 24 == 0) flush_tiles<3, 3>(G, ldg, X, Yt, N, ldx, m);
-  else if (N % 16 == 0) flush_tiles<2, 2>(G, ldg, X, Yt, N, ldx, m);
-  else flush_generic<2>(G, ldg, X, Yt, N, ldx, m);
-}
-
-// The 2N proposals of one slice (LocalK_prop_L: bonds 2N..1, LocalK_prop_R:
-// bonds 1..2N).  Warp 0 evaluates 32 consecutive proposals speculatively
-// against the current G = G0 - X Yt^T; all proposals before the first
-// accepted one are rejections (G and sigma unchanged), so they are exact.
-// One ranf draw per proposal (src/localK.f90:123), advanced in closed form.
-// The slice's sigma (and its neighbours in tau), the Delta table and the
-// plaquette partners are staged in shared memory; warp 0 keeps the ranf state
-// and the acceptance counters in registers for the whole slice.
-__device__ __noinline__ void propose_slice(const ChainDesc &c, const Smem &s, int nt,
-                                           bool descending, int dir) {
-  const int N = c.N, nb = c.nb, k2 = c.k2, Lt = c.Ltrot;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  double *G = s.G;
-  const int ldg = s.ldg;
-  double *X = s.X, *Yt = s.Yt;
-  const int ldx = s.ldx;
-  signed char *sg = c.sigma + (size_t)(nt - 1) * nb;
-  const signed char *gprev = c.sigma + (size_t)((nt - 2 + Lt) % Lt) * nb;
-  const signed char *gnext = c.sigma + (size_t)(nt % Lt) * nb;
-  signed char *sig = s.sig, *sprev = s.sig + nb, *snext = s.sig + 2 * nb;
-  double *dl = s.vec;                                 // [2N][2] Delta(1,1), Delta(1,2)
-  short *bbs = reinterpret_cast<short *>(s.vec + 2 * nb);   // [2N][6]
-  for (int i = threadIdx.x; i < nb; i += Z2_NT) {
-    sig[i] = sg[i];
-    sprev[i] = gprev[i];
-    snext[i] = gnext[i];
-    dl[2 * i] = c.dlt[2 * i];
-    dl[2 * i + 1] = c.dlt[2 * i + 1];
-#pragma unroll
-    for (int q = 0; q < 6; ++q) bbs[6 * i + q] = (short)c.bbonds[6 * i + q];
-  }
-  __syncthreads();
-  double *pdat = s.red + 48;      // accepted proposal: Prod(4), D11, D12, det(Prod)
-  // column pairs of X and Yt as 16-byte words: pair q / 2 of row i
-  const double2 *X2 = reinterpret_cast<const double2 *>(X);
-  const double2 *Y2 = reinterpret_cast<const double2 *>(Yt);
-  const int *__restrict__ bond = s.bond;
-  volatile int *flag = s.flag;
-  unsigned int st = 0;
-  // 48828125^(lane+1) mod 2^31 in a register: lane L draws the (L+1)-th
-  // number of the batch without a divergent constant-memory read
-  const unsigned long long ipl = c_ipow[lane + 1];
-  long long rpos = 0;
-  int den = 0, num = 0;
-  if (warp == 0) {
-    st = *c.rng;
-    if (c.replay) rpos = *c.replay_pos;
-  }
-  int m = 0, done = 0;
-  long long t_eval = 0, t_cols = 0;
-  while (done < nb) {
-    const long long t0 = ph_now();
-    if (warp == 0) {
-      const int kk = done + lane;
-      const bool valid = kk < nb;
-      const int b = valid ? (descending ? nb - 1 - kk : kk) : 0;
-      const int p1 = bond[2 * b], p2 = bond[2 * b + 1];
-      double g11 = G[p1 + (size_t)p1 * ldg], g12 = G[p1 + (size_t)p2 * ldg];
-      double g21 = G[p2 + (size_t)p1 * ldg], g22 = G[p2 + (size_t)p2 * ldg];
-      {
-        // m is even (two columns per accept): two independent FMA chains
-        double h11 = 0.0, h12 = 0.0, h21 = 0.0, h22 = 0.0;
-#pragma unroll 2
-        for (int q = 0; q < m; q += 2) {
-          const size_t o = (size_t)(q >> 1) * ldx;
-          const double2 xa = X2[o + p1], xb = X2[o + p2], ya = Y2[o + p1], yb = Y2[o + p2];
-          g11 -= xa.x * ya.x; g12 -= xa.x * yb.x; g21 -= xb.x * ya.x; g22 -= xb.x * yb.x;
-          h11 += xa.y * ya.y; h12 += xa.y * yb.y; h21 += xb.y * ya.y; h22 += xb.y * yb.y;
-        }
-        g11 -= h11; g12 -= h12; g21 -= h21; g22 -= h22;
-      }
-      const double s_old = (double)sig[b];
-      const double s_new = -s_old;
-      const double D11 = dl[2 * b], D12 = s_new * dl[2 * b + 1];
-      // (I - G)_PP, Prod = I + Delta (I - G)_PP, determinant (no FMA
-      // contraction: same rounding sequence as the reference)
-      const double l11 = __dsub_rn(1.0, g11), l12 = -g12, l21 = -g21, l22 = __dsub_rn(1.0, g22);
-      const double m11 = __dadd_rn(__dmul_rn(D11, l11), __dmul_rn(D12, l21));
-      const double m12 = __dadd_rn(__dmul_rn(D11, l12), __dmul_rn(D12, l22));
-      const double m21 = __dadd_rn(__dmul_rn(D12, l11), __dmul_rn(D11, l21));
-      const double m22 = __dadd_rn(__dmul_rn(D12, l12), __dmul_rn(D11, l22));
-      const double p11 = __dadd_rn(1.0, m11), p12 = m12, p21 = m21, p22 = __dadd_rn(1.0, m22);
-      const double det = __dsub_rn(__dmul_rn(p11, p22), __dmul_rn(p12, p21));
-      // boson ratio (src/fields.f90:40-119) from the host table
-      const short *bb = bbs + 6 * b;
-      const double tmp_old = s_old * sig[bb[0]] * sig[bb[1]] * sig[bb[2]] +
-                             s_old * sig[bb[3]] * sig[bb[4]] * sig[bb[5]];
-      const int is = (int)(-2.0 * tmp_old + 4.0) >> 2;
-      const double tn = s_old * ((double)sprev[b] + (double)snext[b]);
-      const int it = (int)(-2.0 * tn + 4.0) >> 2;
-      const double ratio = __dmul_rn(__dmul_rn(det, det), c.rb[is * 3 + it]);
-      double r;
-      if (c.replay && rpos + lane < c.nreplay) r = c.replay[rpos + lane];
-      else r = (double)(unsigned int)(((unsigned long long)st * ipl) & 0x7fffffffull) *
-               (1.0 / 2147483648.0);
-      const bool acc = valid && (fabs(ratio) > r);
-      const unsigned ball = __ballot_sync(Z2_FULL, acc);
-      const int first = ball ? (__ffs(ball) - 1) : 32;
-      const int rem = nb - done;
-      const int cnt = (first < 32) ? first + 1 : (rem < 32 ? rem : 32);
-      if (lane < cnt && c.dec) {
-        const size_t li = ((size_t)dir * Lt + (nt - 1)) * nb + b;
-        c.dec[li] = (lane == first) ? 1 : 0;
-        if (c.ratios) c.ratios[li] = ratio;
-      }
-      if (lane == first) {
-        // Prod and its determinant; the inverse is formed by the column
-        // phase, where the division overlaps the loads of G, X and Yt
-        pdat[0] = p11; pdat[1] = p12; pdat[2] = p21; pdat[3] = p22;
-        pdat[4] = D11; pdat[5] = D12; pdat[6] = det;
-        flag[1] = b;
-      }
-
-      st = ranf_adv(st, cnt);
-      rpos += cnt;
-      den += cnt;
-      num += (first < 32) ? 1 : 0;
-      __syncwarp();
-      if (lane == 0) {
-        flag[0] = done + cnt;
-        if (first == 32) flag[1] = -1;
-      }
-    }
-    __syncthreads();
-    const long long t1 = ph_now();
-    t_eval += t1 - t0;
-    done = flag[0];
-    const int b = flag[1];
-    if (b >= 0) {
-      const int p1 = bond[2 * b], p2 = bond[2 * b + 1];
-      const double idet = 1.0 / pdat[6];
-      const double q00 = pdat[3] * idet, q01 = -pdat[1] * idet, q10 = -pdat[2] * idet,
-                   q11 = pdat[0] * idet;
-      const double D11 = pdat[4], D12 = pdat[5];
-      for (int i = threadIdx.x; i < N; i += Z2_NT) {
-        double u0 = G[i + (size_t)p1 * ldg], u1 = G[i + (size_t)p2 * ldg];
-        double v0 = G[p1 + (size_t)i * ldg], v1 = G[p2 + (size_t)i * ldg];
-        {
-          // m is even: two independent FMA chains per output
-          double w0 = 0.0, w1 = 0.0, z0 = 0.0, z1 = 0.0;
-#pragma unroll 2
-          for (int q = 0; q < m; q += 2) {
-            const size_t o = (size_t)(q >> 1) * ldx;
-            const double2 xr = X2[o + i], yr = Y2[o + i];
-            const double2 y1 = Y2[o + p1], y2 = Y2[o + p2], x1 = X2[o + p1], x2 = X2[o + p2];
-            u0 -= xr.x * y1.x; u1 -= xr.x * y2.x; v0 -= x1.x * yr.x; v1 -= x2.x * yr.x;
-            w0 += xr.y * y1.y; w1 += xr.y * y2.y; z0 += x1.y * yr.y; z1 += x2.y * yr.y;
-          }
-          u0 -= w0; u1 -= w1; v0 -= z0; v1 -= z1;
-        }
-        // temp = Uhlp * Prodinv ; Vhlp = Delta (I - G)(P, :)
-        const size_t om = (size_t)(m >> 1) * ldx + i;
-        reinterpret_cast<double2 *>(X)[om] = make_double2(u0 * q00 + u1 * q10, u0 * q01 + u1 * q11);
-        double y0 = -D11 * v0 - D12 * v1;
-        double y1 = -D12 * v0 - D11 * v1;
-        if (i == p1) { y0 += D11; y1 += D12; }
-        if (i == p2) { y0 += D12; y1 += D11; }
-        reinterpret_cast<double2 *>(Yt)[om] = make_double2(y0, y1);
-      }
-      if (threadIdx.x == 0) {
-        const signed char sn = (signed char)(-sig[b]);
-        sig[b] = sn;
-        sg[b] = sn;
-      }
-      __syncthreads();
-      t_cols += ph_now() - t1;
-      m += 2;
-      if (m >= k2) {
-        const long long tf = ph_now();
-        rank_update(G, ldg, X, Yt, N, ldx, m, c.flush_shape);
-        m = 0;
-        if (threadIdx.x == 0) c.acc[A_PH0 + PH_FLUSH] += (double)(ph_now() - tf);
-      }
-    }
-  }
-  if (m > 0) {
-    const long long tf = ph_now();
-    rank_update(G, ldg, X, Yt, N, ldx, m, c.flush_shape);
-    if (threadIdx.x == 0) c.acc[A_PH0 + PH_FLUSH] += (double)(ph_now() - tf);
-  }
-  if (threadIdx.x == 0) {
-    *c.rng = st;
-    if (c.replay) *c.replay_pos = rpos;
-    c.acc[A_ACC_DEN] += (double)den;
-    c.acc[A_DRAWS] += (double)den;
-    c.acc[A_ACC_NUM] += (double)num;
-    c.acc[A_PH0 + PH_EVAL] += (double)t_eval;
-    c.acc[A_PH0 + PH_COLS] += (double)t_cols;
-  }
-  __syncthreads();
-}
-
-// ---------------------------------------------------------------------------
 // Equal-time observables (Obs_equal_calc, src/obser_equal.f90:73-149)
 // ---------------------------------------------------------------------------
 __device__ __noinline__ void obs_equal(const ChainDesc &c, const Smem &s, int nt) {
@@ -921,13 +570,13 @@ __device__ __noinline__ void obs_equal(const ChainDesc &c, const Smem &s, int nt
   blk_sum_n<5>(v, s.red);
   if (threadIdx.x == 0) {
     const double flux = v[0] / (double)N;
-    c.acc[A_FLUX_SUM] += flux;
-    c.acc[A_FLUX_SQ] += flux * flux;
-    c.acc[A_PAIR] += v[1];
-    c.acc[A_CDW] += v[2];
-    c.acc[A_CDWS] += v[3];
-    c.acc[A_DENS] += v[4] / (double)N;
-    c.acc[A_NOBS] += 1.0;
+    acc_add(c, A_FLUX_SUM, flux);
+    acc_add(c, A_FLUX_SQ, flux * flux);
+    acc_add(c, A_PAIR, v[1]);
+    acc_add(c, A_CDW, v[2]);
+    acc_add(c, A_CDWS, v[3]);
+    acc_add(c, A_DENS, v[4] / (double)N);
+    acc_add(c, A_NOBS, 1.0);
   }
   __syncthreads();
 }
@@ -998,7 +647,7 @@ struct PhTimer {
   long long t0;
   __device__ PhTimer(const ChainDesc &cc, int p) : c(cc), ph(p), t0(ph_now()) {}
   __device__ ~PhTimer() {
-    if (threadIdx.x == 0) c.acc[A_PH0 + ph] += (double)(ph_now() - t0);
+    if (threadIdx.x == 0) acc_add(c, A_PH0 + ph, (double)(ph_now() - t0));
   }
 };
 

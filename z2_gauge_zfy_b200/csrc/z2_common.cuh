@@ -126,6 +126,16 @@ struct Smem {
   int tile_doubles;
 };
 
+// A pointer into the dynamic shared memory, rebuilt from its base so that the
+// compiler sees the address space (32-bit addresses, ld.shared) of pointers
+// that come out of the Smem table.
+extern __shared__ __align__(16) unsigned char z2_smem[];
+template <class T>
+__device__ __forceinline__ T *as_shared(T *p) {
+  const unsigned off = (unsigned)((size_t)p - (size_t)z2_smem);
+  return reinterpret_cast<T *>(z2_smem + off);
+}
+
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(Z2_FULL, v, o);
@@ -177,6 +187,14 @@ __device__ __forceinline__ void blk_sum_n(double *v, double *red) {
     for (int w = 0; w < Z2_WARPS; ++w) t += red[q * Z2_WARPS + w];
     v[q] = t;
   }
+}
+
+// Adds to one of the chain's counters without waiting for its old value (a
+// reduction at L2; one thread of the chain's block calls it): the load of a
+// plain += stalls that thread, and at the next barrier the block, by an L2
+// round trip.
+__device__ __forceinline__ void acc_add(const ChainDesc &c, int i, double v) {
+  atomicAdd(c.acc + i, v);
 }
 
 __device__ __forceinline__ long long ph_now() { return clock64(); }

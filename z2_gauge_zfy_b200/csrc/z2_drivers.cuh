@@ -405,7 +405,8 @@ __device__ __noinline__ void global_flip_slice(const ChainDesc &c, const Smem &s
     Yt[2 * i + 1] = y1;
   }
   __syncthreads();
-  rank_update(G, ldg, X, Yt, N, ldx, 2);
+  if (c.g_in_smem) rank_update<true>(G, ldg, X, Yt, N, ldx, 2);
+  else rank_update<false>(G, ldg, X, Yt, N, ldx, 2);
   if (threadIdx.x == 0) sg[b] = (signed char)(-sg[b]);
   __syncthreads();
 }
