@@ -328,12 +328,12 @@ static int smem_small_bytes(int N) {
 }
 
 // Shared work space (doubles) a chain keeps after G and the delayed-update
-// factors: the GEMM staging minimum, the pre-pivoted QR's 64-column chunks,
-// and the blocked DORGQR with its parallel T prologue.
+// factors: the GEMM staging minimum, the panel kernels' buffers, and the
+// blocked DORGQR with its parallel T prologue.
 static size_t tile_min(int N) {
-  const int ldv = qrf_ldv(N);
+  const int ldv = ((N + 11) & ~15) + 4;
   size_t t = kGemmTile;
-  t = std::max<size_t>(t, qrf_min_work(N));
+  t = std::max<size_t>(t, wy_work(N));
   t = std::max<size_t>(t, (size_t)ldv * 16 + 17 * (size_t)std::max(N - 16, 0));
   t = std::max<size_t>(t, (size_t)Z2_WARPS * (2 * 16 * 16 + 4 * 16));
   return t;

@@ -2,6 +2,7 @@
 // evaluated at once, accepted flips queued as rank-2 factors and flushed as
 // one rank-2k DMMA update.
 #pragma once
+#include "z2_blocked.cuh"
 #include "z2_flush.cuh"
 
 // 48828125^n mod 2^31 (the ranf multiplier power of the n-th draw): the low 32
@@ -13,16 +14,6 @@ __device__ __forceinline__ unsigned int ranf_pow(int n) {
     p *= p;
   }
   return m & 0x7fffffffu;
-}
-
-// 1 / x to rounding for a normal x of moderate size: the hardware's
-// approximation and two Newton steps r <- r (2 - x r) (no special cases, so it
-// schedules beside other work, unlike the division).
-__device__ __forceinline__ double rcp_newton(double x) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  r = fma(r, fma(-x, r, 1.0), r);
-  return fma(r, fma(-x, r, 1.0), r);
 }
 
 // LocalK_prop_L / LocalK_prop_R's proposals (src/localK.f90:45-173): bonds
