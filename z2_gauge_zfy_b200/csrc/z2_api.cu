@@ -95,9 +95,9 @@ z2_unit_kernel(const ChainDesc *desc, int op, UnitArgs a, unsigned smem_bytes) {
     dev_stab_green(s, N, a.nt, sc.Ltrot, a.UR, a.DR, a.VR, a.ULT, a.DL, a.VL, A, lda, sc.W1,
                    sc.W2, sc.W0, a.G);
   } else if (op == U_STAB_GREEN_BIG) {
-    dev_stab_green_big(s, N, a.UR, a.DR, a.VR, a.ULT, a.DL, a.VL, sc.W0, sc.W1, sc.W2, sc.W3,
-                       sc.B0, sc.B1, sc.B2, sc.B3);
-    green_big_extract(N, sc.B3, a.G, a.G0t, a.Gt0, a.Gtt);
+    int lda; double *A = qr_matrix(sc, s, lda);
+    dev_stab_green_big(s, N, a.UR, a.DR, a.VR, a.ULT, a.DL, a.VL, A, lda, sc.W0, sc.W1, sc.W2, sc.W3,
+                       a.G, a.G0t, a.Gt0, a.Gtt);
   }
 }
 
@@ -109,7 +109,6 @@ namespace {
 const double kZero = 1.0e-10;      // src/calc_basic.f90:5
 const double kUpbound = 1.0e200;   // src/calc_basic.f90:7
 const int kSmemMax = 227 * 1024 - 2048;
-const int kGemmTile = Z2_MIN_TILE;
 
 int npbc(int nr, int L) { return nr < 1 ? nr + L : (nr > L ? nr - L : nr); }
 
@@ -328,16 +327,9 @@ static int smem_small_bytes(int N) {
 }
 
 // Shared work space (doubles) a chain keeps after G and the delayed-update
-// factors: the GEMM staging minimum, the panel kernels' buffers, and the
-// blocked DORGQR with its parallel T prologue.
-static size_t tile_min(int N) {
-  const int ldv = ((N + 11) & ~15) + 4;
-  size_t t = kGemmTile;
-  t = std::max<size_t>(t, wy_work(N));
-  t = std::max<size_t>(t, (size_t)ldv * 16 + 17 * (size_t)std::max(N - 16, 0));
-  t = std::max<size_t>(t, (size_t)Z2_WARPS * (2 * 16 * 16 + 4 * 16));
-  return t;
-}
+// factors: the panel kernels' buffers (which also cover the pivoted QR's 2 N
+// and the blocked LU's 16 x 16).
+static size_t tile_min(int N) { return std::max<size_t>(512, wy_work(N)); }
 
 // Delayed-update rank when the caller names none: the columns of an accept
 // cost a loop over the queued pairs, a flush its fragment loads.  Cycles per
@@ -521,7 +513,7 @@ extern "C" int z2_create(z2_handle **out, const z2_chain_params *params, int32_t
     size_t o_stv = take(8 * (size_t)N * 2 * (Nst + 1));
     size_t o_tau = take(8 * NN * 8);              // G00, Gtt, Gt0, G0t, URd, VRd, ULTd, VLd
     size_t o_tauv = take(8 * (size_t)N * 2);      // DRd, DLd
-    size_t o_big = take(8 * NN * 16);             // B0..B3 (2N x 2N)
+    size_t o_big = take(8 * NN * 3);              // T0..T2
     size_t o_otau = take(8 * (size_t)7 * Lt * N);
     size_t o_grad = take(8 * (size_t)nb);
     size_t o_acc = take(8 * A_COUNT);
@@ -609,7 +601,7 @@ extern "C" int z2_create(z2_handle **out, const z2_chain_params *params, int32_t
     double *tv = (double *)(base + o_tauv);
     d.DRd = tv; d.DLd = tv + N;
     double *bg = (double *)(base + o_big);
-    d.B0 = bg; d.B1 = bg + 4 * NN; d.B2 = bg + 8 * NN; d.B3 = bg + 12 * NN;
+    d.T0 = bg; d.T1 = bg + NN; d.T2 = bg + 2 * NN;
     d.obs_tau = (double *)(base + o_otau);
     d.grad = (double *)(base + o_grad);
     d.acc = (double *)(base + o_acc);

@@ -422,103 +422,52 @@ __device__ __noinline__ void apply_pending_L(const ChainDesc &c, const Smem &s, 
 // ---------------------------------------------------------------------------
 // Stabilization (src/stabilization.f90:42-264)
 // ---------------------------------------------------------------------------
-// stab_green_big (src/stabilization.f90:202-264): the four blocks of the
-// 2N x 2N Green's function.  Inverses of the orthogonal factors (UL UR,
-// bigU, UR, UL) are their transposes; VR VL, VR and VL are inverted by LU;
-// bigV (triangular) by a triangular solve.  The 2N x 2N QR (UDV_C) is the
-// blocked Householder QR, bigU the blocked DORGQR, products DMMA GEMMs.
+// stab_green_big (src/stabilization.f90:202-264): G(0,0), G(0,tau), G(tau,0),
+// G(tau,tau) from the UDV factors of the two products.  The reference inverts a
+// 2N x 2N matrix (its QR, the inverses of VR VL, VR, VL and bigV); the four
+// blocks all contain the inverse of the same N x N middle matrix as stab_green:
+// with B_tau..B_1 = UR DR VR, B_L..B_tau+1 = VL DL UL and
+//   M' = DRb^-1 (UR^T UL^T) DLb^-1 + DRs (VR VL) DLs   (z2_stab.cuh)
+//   G(tau,tau) = UL^T DLb^-1 M'^-1 DRb^-1 UR^T,   G(tau,0) = UL^T DLb^-1 M'^-1 DRs VR,
+//   G(0,tau) = -VL DLs M'^-1 DRb^-1 UR^T,         G(0,0) = 1 - VL DLs M'^-1 DRs VR,
+// every factor of order one, scales only divided out: one inverse and eight
+// N x N x N products (at N = 100, 0.5 M cycles against 9 M for the 2N x 2N QR).
+// M (ldm): work matrix (shared arena when it fits); W0..W3 N x N global
+// workspaces; outputs N x N (ld N).
 __device__ __noinline__ void dev_stab_green_big(const Smem &s, int N, const double *UR, const double *DR,
                                    const double *VR, const double *ULT, const double *DL,
-                                   const double *VL, double *W0, double *W1, double *W2,
-                                   double *W3, double *B0, double *B1, double *B2, double *B3) {
-  const int n2 = 2 * N;
-  double *tau = s.vec;          // 2N
-  double *bigD = s.vec + 2 * N; // 2N
-  int *ipiv = s.ivec;
-  // invVRVL = (VR VL)^-1  -> W0
-  {
-    blk_dmma(N, N, N, 1.0, MatRef{VR, 1, N}, false, MatRef{VL, 1, N}, false, 0.0, W0, N);
-    blk_inverse_blocked(W0, N, N, W1, N, ipiv, s.red, s.flag, s.tile,
-                        s.tile_doubles);
-  }
-  // invULUR = UR^T UL^T -> W1
-  {
-    blk_dmma(N, N, N, 1.0, MatRef{UR, N, 1}, false, MatRef{ULT, 1, N}, false, 0.0, W1, N);
-  }
-  // big matrix
-  for (int j = threadIdx.x / 32; j < n2; j += Z2_WARPS)
-    for (int i = threadIdx.x & 31; i < n2; i += 32) {
-      double v = 0.0;
-      if (i < N && j < N) v = W0[i + (size_t)j * N];
-      else if (i >= N && j >= N) v = W1[(i - N) + (size_t)(j - N) * N];
-      else if (i < N && j == i + N) v = DL[i];
-      else if (i >= N && j == i - N) v = -DR[j];
-      B0[i + (size_t)j * n2] = v;
-    }
-  __syncthreads();
-  // UDV_C: QR, D = |R_ii|, V = R / D, determinant-sign fix
-  blk_geqrf(B0, n2, n2, tau, s.tile, s.tile_doubles, s.vec + 4 * N, 4 * N, s.red);
-  blk_copy(B1, n2, B0, n2, n2, n2);
-  blk_orgqr(B1, n2, n2, tau, s.tile, s.tile_doubles, s.vec + 4 * N, 4 * N);   // bigU
-  {
-    // sign of prod R_ii (mat_mod.f90:650-657): count negative diagonals
-    int neg = 0;
-    for (int i = threadIdx.x; i < n2; i += Z2_NT) neg += (B0[i + (size_t)i * n2] < 0.0);
-    double t = blk_sum((double)neg, s.red);
-    int flip = ((int)t) & 1;
-    for (int i = threadIdx.x; i < n2; i += Z2_NT) bigD[i] = fabs(B0[i + (size_t)i * n2]);
-    __syncthreads();
-    // bigV = R / D (upper), into B2 ; flip row 0 of V and column 0 of U if needed
-    for (int j = threadIdx.x / 32; j < n2; j += Z2_WARPS)
-      for (int i = threadIdx.x & 31; i < n2; i += 32) {
-        double v = (i <= j) ? B0[i + (size_t)j * n2] : 0.0;
-        if (flip && i == 0) v = -v;
-        B2[i + (size_t)j * n2] = v / bigD[i];
-      }
-    if (flip)
-      for (int i = threadIdx.x; i < n2; i += Z2_NT) B1[i] = -B1[i];
-    __syncthreads();
-  }
-  // invbigV: solve bigV X = I -> B3
-  blk_identity(B3, n2, n2);
-  blk_trsm_lun_blocked(B2, n2, n2, B3, n2, n2);
-  // invVUR -> W2, invVUL -> W3
-  blk_copy(W2, N, VR, N, N, N);
-  blk_inverse_blocked(W2, N, N, W0, N, ipiv, s.red, s.flag, s.tile,
-                        s.tile_doubles);
-  blk_copy(W3, N, VL, N, N, N);
-  blk_inverse_blocked(W3, N, N, W0, N, ipiv, s.red, s.flag, s.tile,
-                        s.tile_doubles);
-  // mat_left = diag(invVUR, invUUL) invbigV -> B0
-  {
-    blk_dmma(N, n2, N, 1.0, MatRef{W2, 1, N}, false, MatRef{B3, 1, n2}, false, 0.0, B0, n2);
-    blk_dmma(N, n2, N, 1.0, MatRef{ULT, 1, N}, false, MatRef{B3 + N, 1, n2}, false, 0.0, B0 + N, n2);
-  }
-  // mat_right = invbigU diag(invVUL, invUUR) -> B2 ; invbigU = bigU^T
-  {
-    blk_dmma(n2, N, N, 1.0, MatRef{B1, n2, 1}, false, MatRef{W3, 1, N}, false, 0.0, B2, n2);
-    blk_dmma(n2, N, N, 1.0, MatRef{B1 + N, n2, 1}, false, MatRef{UR, N, 1}, false, 0.0,
-             B2 + (size_t)N * n2, n2);
-  }
-  // mat_left(:, nr) /= bigD(nr)
-  for (int j = threadIdx.x / 32; j < n2; j += Z2_WARPS) {
-    double d = bigD[j];
-    for (int i = threadIdx.x & 31; i < n2; i += 32) B0[i + (size_t)j * n2] = B0[i + (size_t)j * n2] / d;
+                                   const double *VL, double *M, int ldm, double *W0, double *W1,
+                                   double *W2, double *W3, double *G00, double *G0t, double *Gt0,
+                                   double *Gtt) {
+  double *rRb = s.vec + N, *rLb = s.vec + 2 * N, *neg = s.vec + 5 * N;
+  int *piv = s.ivec, *inv = s.ivec + N;
+  middle_inverse(s, N, UR, DR, VR, ULT, DL, VL, M, ldm, rRb, rLb, s.vec + 3 * N, s.vec + 4 * N, piv, W0,
+                 W1);
+  for (int m = threadIdx.x; m < N; m += Z2_NT) {
+    inv[piv[m]] = m;
+    neg[m] = -1.0;
   }
   __syncthreads();
-  {
-    blk_dmma(n2, n2, n2, 1.0, MatRef{B0, 1, n2}, false, MatRef{B2, 1, n2}, false, 0.0, B3, n2);
-  }
-}
-
-// Blocks of the 2N x 2N Green's function left in B3 by dev_stab_green_big.
-__device__ __noinline__ void green_big_extract(int N, const double *B3, double *G00, double *G0t,
-                                  double *Gt0, double *Gtt) {
-  const int n2 = 2 * N;
-  blk_copy(G00, N, B3, n2, N, N);
-  blk_copy(G0t, N, B3 + (size_t)N * n2, n2, N, N);
-  blk_copy(Gt0, N, B3 + N, n2, N, N);
-  blk_copy(Gtt, N, B3 + N + (size_t)N * n2, n2, N, N);
+  // DLb^-1 M'^-1 DRb^-1 UR^T -> W1; the columns of M times DR (DRs = DRb^-1 DR):
+  // DLb^-1 M'^-1 DRs VR -> W2
+  permute_cols(M, ldm, N, inv, rRb, W0);
+  gemm_nnn(N, MatRef{M, 1, ldm}, piv, false, MatRef{UR, N, 1}, false, GemmOut{W1, N, rLb});
+  blk_scale_cols(M, ldm, N, N, DR);
+  gemm_nnn(N, MatRef{M, 1, ldm}, piv, false, MatRef{VR, 1, N}, false, GemmOut{W2, N, rLb});
+  gemm_nnn(N, MatRef{ULT, 1, N}, nullptr, false, MatRef{W1, 1, N}, false, GemmOut{Gtt, N});
+  gemm_nnn(N, MatRef{ULT, 1, N}, nullptr, false, MatRef{W2, 1, N}, false, GemmOut{Gt0, N});
+  // DLs = DLb^-1 DL
+  blk_walk<4, double2>(
+      N, N, [&](int i, int j) { return make_double2(W1[i + (size_t)j * N], W2[i + (size_t)j * N]); },
+      [&](double2 v, int i, int j) {
+        W0[i + (size_t)j * N] = v.x * DL[i];
+        W3[i + (size_t)j * N] = v.y * DL[i];
+      });
+  __syncthreads();
+  gemm_nnn(N, MatRef{VL, 1, N}, nullptr, false, MatRef{W0, 1, N}, false, GemmOut{G0t, N, neg});
+  gemm_nnn(N, MatRef{VL, 1, N}, nullptr, false, MatRef{W3, 1, N}, false, GemmOut{G00, N, neg});
+  for (int i = threadIdx.x; i < N; i += Z2_NT) G00[i + (size_t)i * N] += 1.0;
+  __syncthreads();
 }
 
 // ---------------------------------------------------------------------------

@@ -12,7 +12,6 @@
 #define Z2_WARPS (Z2_NT / 32)
 #define Z2_FULL 0xffffffffu
 #define Z2_NRED 64              // doubles of block-reduction scratch
-#define Z2_MIN_TILE 2080        // doubles of shared work space kept after G and X, Y
 
 // Accumulator layout of ChainDesc::acc (doubles).
 enum {
@@ -82,7 +81,7 @@ struct ChainDesc {
   // time-displaced chain
   double *G00, *Gtt, *Gt0, *G0t;
   double *URd, *VRd, *DRd, *ULTd, *VLd, *DLd;
-  double *B0, *B1, *B2, *B3;                      // 2N x 2N workspaces
+  double *T0, *T1, *T2;                           // N x N workspaces of stab_green_big
   double *obs_tau;      // [7][Ltrot][N]
   double *grad;         // [2N] adjoint output
   // global moves: state backup (G..VL, DR DL, stacks, Xmaxm), cluster mask

@@ -223,7 +223,7 @@ __device__ __noinline__ void blk_geqp3_tc(double *A, int lda, int n, int *jpvt, 
       int oi = __shfl_xor_sync(Z2_FULL, bi, o);
       if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
     }
-    const int pvt = bi;
+    const int pvt = bi < n ? bi : j;   // no candidate: a column of NaNs
     __syncthreads();
     if (warp == 0) {
       double *Aj = A + (size_t)j * lda;
@@ -305,338 +305,6 @@ __device__ __noinline__ void blk_org2r_tc(double *A, int lda, int m, int n, cons
   }
 }
 
-// T of one block of reflectors (DLARFT forward / columnwise), by one warp:
-// T is the inverse of the upper-triangular matrix with diagonal 1/tau and
-// strict upper part S = V^T V (DLARFT's column recurrence is exactly the
-// forward substitution of that inverse); diagonal blocks of size b pair up
-// as T12 = -T11 S12 T22, four levels of short dot products instead of 16
-// dependent columns.  A zero tau zeroes its row and column, as in DLARFT.
-// S, T: ib x ib (ld ib); tb: the block's tau; Xs: 4 ib doubles of scratch.
-__device__ __forceinline__ void warp_larft_t(const double *S, double *T, int ib, const double *tb,
-                                             double *Xs) {
-  const int lane = threadIdx.x & 31;
-  for (int e = lane; e < ib * ib; e += 32) {
-    const int r = e % ib, c = e / ib;
-    T[e] = (r == c) ? tb[c] : 0.0;
-  }
-  __syncwarp();
-  for (int b = 1; b < ib; b <<= 1) {
-    const int np = (ib + 2 * b - 1) / (2 * b), bb = b * b;
-    for (int e = lane; e < np * bb; e += 32) {
-      const int p = e / bb, r = (e % bb) % b, c = (e % bb) / b;
-      const int k = 2 * b * p, k2 = k + b;
-      if (k2 + c < ib) {
-        double x0 = 0.0, x1 = 0.0;
-        for (int q = 0; q <= c; q += 2) {
-          x0 += S[(k + r) + (k2 + q) * ib] * T[(k2 + q) + (k2 + c) * ib];
-          if (q + 1 <= c) x1 += S[(k + r) + (k2 + q + 1) * ib] * T[(k2 + q + 1) + (k2 + c) * ib];
-        }
-        Xs[e] = x0 + x1;
-      }
-    }
-    __syncwarp();
-    for (int e = lane; e < np * bb; e += 32) {
-      const int p = e / bb, r = (e % bb) % b, c = (e % bb) / b;
-      const int k = 2 * b * p, k2 = k + b;
-      if (k2 + c < ib) {
-        double t0 = 0.0, t1 = 0.0;
-        for (int q = r; q < b; q += 2) {
-          t0 += T[(k + r) + (k + q) * ib] * Xs[p * bb + q + c * b];
-          if (q + 1 < b) t1 += T[(k + r) + (k + q + 1) * ib] * Xs[p * bb + q + 1 + c * b];
-        }
-        T[(k + r) + (k2 + c) * ib] = -(t0 + t1);
-      }
-    }
-    __syncwarp();
-  }
-}
-
-// S = V^T V (ib x ib, ld ib, ib <= 16) for the unit lower trapezoidal V of
-// the reflectors stored in A(i0:n, i0:i0+ib), by one warp: one 16 x 16 DMMA
-// group over k = n - i0, the operand read from A with the unit diagonal and
-// zero upper part applied (the same k order and values as blk_dmma on a
-// copy of V, so the same bits).
-__device__ __forceinline__ void warp_gram_v(const double *A, int lda, int n, int i0, int ib, double *S) {
-  const int lane = threadIdx.x & 31, lr = lane >> 2, lc = lane & 3;
-  const int mp = n - i0;
-  auto vat = [&](int l, int c) -> double {
-    if (l >= mp || c >= ib) return 0.0;
-    return (l == c) ? 1.0 : (l > c ? A[(i0 + l) + (size_t)(i0 + c) * lda] : 0.0);
-  };
-  double acc[2][2][2] = {};
-  for (int l0 = 0; l0 < mp; l0 += 4) {
-    const double f0 = vat(l0 + lc, lr), f1 = vat(l0 + lc, 8 + lr);
-    dmma884(acc[0][0][0], acc[0][0][1], f0, f0);
-    dmma884(acc[0][1][0], acc[0][1][1], f0, f1);
-    dmma884(acc[1][0][0], acc[1][0][1], f1, f0);
-    dmma884(acc[1][1][0], acc[1][1][1], f1, f1);
-  }
-#pragma unroll
-  for (int u = 0; u < 2; ++u)
-#pragma unroll
-    for (int v = 0; v < 2; ++v)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int r = 8 * u + lr, c = 8 * v + 2 * lc + e;
-        if (r < ib && c < ib) S[r + c * ib] = 1.0 * acc[u][v][e];
-      }
-}
-
-// DORGQR for a square n x n matrix with n reflectors, blocked: blocks of nb
-// reflectors from the last to the first, each applied as the compact WY form
-// H_i0 ... H_i0+ib-1 = I - V T V^T (DLARFT forward/columnwise) by DMMA GEMMs:
-//   trailing columns  C <- C - V (T (V^T C)),
-//   block columns     A(i0:, i0:i0+ib) = E - V (T V1^T),  rows above = 0.
-// work (shared memory, wd doubles) holds V (ldv x nb, ldv = 4 mod 16 so both
-// DMMA fragment orientations are bank-conflict free) and W (ldw x (n - nb),
-// ldw odd for the thread-per-column T W product); T and the Gram matrix
-// (nb x nb each) go to small (sd doubles) when it is large enough, else to
-// work.  When work is too small the unblocked DORG2R runs instead (same Q up
-// to rounding).
-__device__ __noinline__ void blk_orgqr(double *A, int lda, int n, const double *tau, double *work,
-                                      int wd, double *small, int sd, double *tscr = nullptr) {
-  const int ldv = ((n + 11) & ~15) + 4;
-  int nb = 16;
-  auto need = [n, ldv, sd](int b) {
-    return ldv * b + (b + 1) * (n > b ? n - b : 0) + (2 * b * b <= sd ? 0 : 2 * b * b);
-  };
-  if (need(nb) > wd) nb = 8;
-  if (need(nb) > wd) {
-    blk_org2r_tc(A, lda, n, n, tau);
-    return;
-  }
-  const int ldw = nb + 1;
-  double *V = work;
-  double *W = V + (size_t)ldv * nb;
-  double *T = (2 * nb * nb <= sd) ? small : W + (size_t)ldw * (n > nb ? n - nb : 0);
-  double *S = T + nb * nb;
-  const int tid = threadIdx.x;
-  // Prologue (tscr: nb^2 ceil(n / nb) doubles of global scratch): the T of
-  // every block depends only on that block's reflectors, which the backward
-  // loop below does not touch before the block's turn, so all of them are
-  // formed first, one warp per block in parallel, instead of one after the
-  // other inside the loop.
-  if (tscr != nullptr && wd < Z2_WARPS * (2 * nb * nb + 4 * nb)) tscr = nullptr;
-  if (tscr != nullptr) {
-    const int nblk = (n + nb - 1) / nb, warp = tid >> 5;
-    double *Sw = work + (size_t)warp * (2 * nb * nb + 4 * nb);
-    double *Tw = Sw + nb * nb, *Xw = Tw + nb * nb;
-    for (int bi = warp; bi < nblk; bi += Z2_WARPS) {
-      const int i0 = bi * nb, ib = (n - i0) < nb ? (n - i0) : nb;
-      warp_gram_v(A, lda, n, i0, ib, Sw);
-      __syncwarp();
-      warp_larft_t(Sw, Tw, ib, tau + i0, Xw);
-      __syncwarp();
-      double *td = tscr + (size_t)bi * nb * nb;
-      for (int e = tid & 31; e < ib * ib; e += 32) td[e] = Tw[e];
-      __syncwarp();
-    }
-    __syncthreads();
-  }
-  for (int i0 = ((n - 1) / nb) * nb; i0 >= 0; i0 -= nb) {
-    const int ib = (n - i0) < nb ? (n - i0) : nb;
-    const int mp = n - i0, nc = n - i0 - ib;
-    // V: unit lower trapezoidal, mp x ib
-    for (int c = tid >> 5; c < ib; c += Z2_WARPS)
-      for (int r = tid & 31; r < mp; r += 32)
-        V[r + (size_t)c * ldv] = (r == c) ? 1.0 : (r > c ? A[(i0 + r) + (size_t)(i0 + c) * lda] : 0.0);
-    __syncthreads();
-    // S = V^T V (the prologue already folded it into T)
-    if (tscr == nullptr)
-      blk_dmma(ib, ib, mp, 1.0, MatRef{V, ldv, 1}, false, MatRef{V, 1, ldv}, false, 0.0, S, ib);
-    // T (DLARFT): from the prologue when it ran, else by one warp here
-    if (tscr != nullptr) {
-      const double *tsrc = tscr + (size_t)(i0 / nb) * nb * nb;
-      for (int e = tid; e < ib * ib; e += Z2_NT) T[e] = tsrc[e];
-    } else if (ldw * (n - nb) >= 4 * nb) {
-      if (tid < 32) warp_larft_t(S, T, ib, tau + i0, W);
-    } else if (tid < ib) {
-      const int r = tid;
-      double tr[16];
-#pragma unroll
-      for (int c = 0; c < 16; ++c) {
-        double t = 0.0;
-        if (c < ib) {
-          if (c == r) {
-            t = tau[i0 + c];
-          } else if (c > r) {
-            double a0 = 0.0, a1 = 0.0;
-#pragma unroll
-            for (int q = 0; q < c; ++q) {
-              if (q >= r) {
-                if (q & 1) a1 += tr[q] * S[q + c * ib];
-                else a0 += tr[q] * S[q + c * ib];
-              }
-            }
-            t = -tau[i0 + c] * (a0 + a1);
-          }
-        }
-        tr[c] = t;
-      }
-#pragma unroll
-      for (int c = 0; c < 16; ++c)
-        if (c < ib) T[r + c * ib] = tr[c];
-    }
-    __syncthreads();
-    if (nc > 0) {
-      double *C = A + i0 + (size_t)(i0 + ib) * lda;
-      // W = V^T C  (ib x nc, ld ldw)
-      blk_dmma(ib, nc, mp, 1.0, MatRef{V, ldv, 1}, false, MatRef{C, 1, lda}, false, 0.0, W, ldw);
-      // W <- T W, one thread per column
-      for (int j = tid; j < nc; j += Z2_NT) {
-        double w[16];
-#pragma unroll
-        for (int q = 0; q < 16; ++q) w[q] = (q < ib) ? W[q + j * ldw] : 0.0;
-#pragma unroll
-        for (int r = 0; r < 16; ++r) {
-          if (r < ib) {
-            double t = 0.0;
-#pragma unroll
-            for (int q = r; q < 16; ++q)
-              if (q < ib) t += T[r + q * ib] * w[q];
-            W[r + j * ldw] = t;
-          }
-        }
-      }
-      __syncthreads();
-      // C -= V W
-      blk_dmma(mp, nc, ib, -1.0, MatRef{V, 1, ldv}, false, MatRef{W, 1, ldw}, false, 1.0, C, lda);
-    }
-    // S <- T V1^T (ib x ib); block columns <- E - V S, rows above i0 <- 0
-    for (int e = tid; e < ib * ib; e += Z2_NT) {
-      const int r = e % ib, c = e / ib;
-      double t = 0.0;
-      for (int q = r; q <= c; ++q) t += T[r + q * ib] * V[c + (size_t)q * ldv];
-      S[r + c * ib] = t;
-    }
-    for (int c = tid >> 5; c < ib; c += Z2_WARPS)
-      for (int r = tid & 31; r < n; r += 32) A[r + (size_t)(i0 + c) * lda] = (r == i0 + c) ? 1.0 : 0.0;
-    __syncthreads();
-    blk_dmma(mp, ib, ib, -1.0, MatRef{V, 1, ldv}, false, MatRef{S, 1, ib}, false, 1.0,
-             A + i0 + (size_t)i0 * lda, lda);
-  }
-}
-
-// Householder QR without pivoting of a square n x n matrix, blocked (DGEQRF
-// structure): panels of nb columns are factored column by column (DLARFG on
-// the column, the reflector applied to the rest of the panel one warp per
-// column), then the panel's reflectors reach the trailing columns as
-// C <- (I - V T^T V^T) C = C - V (T^T (V^T C)) by DMMA GEMMs (T by DLARFT's
-// recurrence, as in blk_orgqr).  Same R, tau and reflectors as DGEQR2 up to
-// rounding.  Workspace as blk_orgqr; falls back to blk_geqr2 when short.
-__device__ __noinline__ void blk_geqrf(double *A, int lda, int n, double *tau, double *work, int wd,
-                                      double *small, int sd, double *red) {
-  const int ldv = ((n + 11) & ~15) + 4;
-  int nb = 16;
-  auto need = [n, ldv, sd](int b) {
-    return ldv * b + (b + 1) * (n > b ? n - b : 0) + (2 * b * b <= sd ? 0 : 2 * b * b);
-  };
-  if (need(nb) > wd) nb = 8;
-  if (need(nb) > wd) {
-    blk_geqr2(A, lda, n, n, tau);
-    return;
-  }
-  const int ldw = nb + 1;
-  double *V = work;
-  double *W = V + (size_t)ldv * nb;
-  double *T = (2 * nb * nb <= sd) ? small : W + (size_t)ldw * (n > nb ? n - nb : 0);
-  double *S = T + nb * nb;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int j0 = 0; j0 < n; j0 += nb) {
-    const int ib = (n - j0) < nb ? (n - j0) : nb;
-    const int mp = n - j0, nc = n - j0 - ib;
-    // ---- panel (DGEQR2 on columns j0 .. j0+ib-1) ----
-    for (int k = 0; k < ib; ++k) {
-      const int j = j0 + k;
-      double *Aj = A + (size_t)j * lda;
-      double ss = 0.0;
-      for (int r = j + 1 + tid; r < n; r += Z2_NT) { const double a = Aj[r]; ss += a * a; }
-      ss = blk_sum(ss, red);
-      const double alpha = Aj[j];
-      double t = 0.0, beta = alpha, sc = 1.0;
-      if (j < n - 1 && ss != 0.0) {
-        const double xnorm = sqrt(ss);
-        beta = -copysign(dlapy2(alpha, xnorm), alpha);
-        t = (beta - alpha) / beta;
-        sc = 1.0 / (alpha - beta);
-      }
-      if (t != 0.0)
-        for (int r = j + 1 + tid; r < n; r += Z2_NT) Aj[r] *= sc;
-      __syncthreads();
-      // H_j on the remaining panel columns, one warp per column (v_j = 1)
-      if (t != 0.0) {
-        for (int c = j + 1 + warp; c < j0 + ib; c += Z2_WARPS) {
-          double *Ac = A + (size_t)c * lda;
-          const double acj = Ac[j];
-          double w = 0.0;
-          for (int r = j + 1 + lane; r < n; r += 32) w += Aj[r] * Ac[r];
-          w = (warp_sum(w) + acj) * t;
-          __syncwarp();
-          if (lane == 0) Ac[j] = acj - w;
-          for (int r = j + 1 + lane; r < n; r += 32) Ac[r] -= w * Aj[r];
-        }
-      }
-      __syncthreads();
-      if (tid == 0) { tau[j] = t; Aj[j] = beta; }
-      __syncthreads();
-    }
-    if (nc <= 0) continue;
-    // ---- V (unit lower), S = V^T V, T (DLARFT) ----
-    for (int c = tid >> 5; c < ib; c += Z2_WARPS)
-      for (int r = tid & 31; r < mp; r += 32)
-        V[r + (size_t)c * ldv] = (r == c) ? 1.0 : (r > c ? A[(j0 + r) + (size_t)(j0 + c) * lda] : 0.0);
-    __syncthreads();
-    blk_dmma(ib, ib, mp, 1.0, MatRef{V, ldv, 1}, false, MatRef{V, 1, ldv}, false, 0.0, S, ib);
-    if (tid < ib) {
-      const int r = tid;
-      double tr[16];
-#pragma unroll
-      for (int c = 0; c < 16; ++c) {
-        double t = 0.0;
-        if (c < ib) {
-          if (c == r) {
-            t = tau[j0 + c];
-          } else if (c > r) {
-            double a0 = 0.0, a1 = 0.0;
-#pragma unroll
-            for (int q = 0; q < c; ++q) {
-              if (q >= r) {
-                if (q & 1) a1 += tr[q] * S[q + c * ib];
-                else a0 += tr[q] * S[q + c * ib];
-              }
-            }
-            t = -tau[j0 + c] * (a0 + a1);
-          }
-        }
-        tr[c] = t;
-      }
-#pragma unroll
-      for (int c = 0; c < 16; ++c)
-        if (c < ib) T[r + c * ib] = tr[c];
-    }
-    __syncthreads();
-    // ---- trailing columns: C -= V (T^T (V^T C)) ----
-    double *C = A + j0 + (size_t)(j0 + ib) * lda;
-    blk_dmma(ib, nc, mp, 1.0, MatRef{V, ldv, 1}, false, MatRef{C, 1, lda}, false, 0.0, W, ldw);
-    for (int c = tid; c < nc; c += Z2_NT) {
-      double w[16];
-#pragma unroll
-      for (int q = 0; q < 16; ++q) w[q] = (q < ib) ? W[q + c * ldw] : 0.0;
-#pragma unroll
-      for (int r = 0; r < 16; ++r) {
-        if (r < ib) {
-          double t = 0.0;
-#pragma unroll
-          for (int q = 0; q <= r; ++q) t += T[q + r * ib] * w[q];   // (T^T w)_r
-          W[r + c * ldw] = t;
-        }
-      }
-    }
-    __syncthreads();
-    blk_dmma(mp, nc, ib, -1.0, MatRef{V, 1, ldv}, false, MatRef{W, 1, ldw}, false, 1.0, C, lda);
-  }
-}
-
 // Solve L Z = Y in place, L unit lower triangular (below the diagonal of L),
 // Y n x nc: blocks of 8 rows from the top, the 8 x 8 diagonal block solved one
 // thread per column in registers, the rows below updated by DMMA.
@@ -683,14 +351,9 @@ __device__ __noinline__ void blk_trsm_lun_blocked(const double *R, int ldr, int 
 // one thread per column (L11 staged in work), A22 -= L21 U12 by DMMA; then
 // A^-1 = U^-1 L^-1 P from the identity by the two blocked triangular solves.
 // A is overwritten by its inverse; W (ldw) is an n x n workspace; work holds
-// >= 256 doubles of shared memory (else the unblocked blk_inverse runs).
+// 256 doubles of shared memory.
 __device__ __noinline__ void blk_inverse_blocked(double *A, int lda, int n, double *W, int ldw,
-                                                 int *ipiv, double *red, int *flag, double *work,
-                                                 int wd) {
-  if (work == nullptr || wd < 256) {
-    blk_inverse(A, lda, n, W, ldw, ipiv, red, flag);
-    return;
-  }
+                                                 int *ipiv, double *red, int *flag, double *work) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int j0 = 0; j0 < n; j0 += 16) {
     const int jb = (n - j0) < 16 ? (n - j0) : 16;
@@ -711,7 +374,7 @@ __device__ __noinline__ void blk_inverse_blocked(double *A, int lda, int n, doub
       bv = red[0]; bi = flag[0];
       for (int w = 1; w < Z2_WARPS; ++w)
         if (red[w] > bv || (red[w] == bv && flag[w] < bi)) { bv = red[w]; bi = flag[w]; }
-      const int p = bi;
+      const int p = bi < n ? bi : k;   // no candidate: a column of NaNs
       __syncthreads();
       if (tid == 0) ipiv[k] = p;
       if (p != k)

@@ -5,7 +5,7 @@
 
 // Wrap_tau (src/stabilization.f90:478-514) on the Dyn copy of the propagator.
 __device__ __noinline__ void wrap_tau(const ChainDesc &c, const Smem &s, int nt, Pend &pd) {
-  const int N = c.N, NN = N * N, n2 = 2 * N;
+  const int N = c.N, NN = N * N;
   int lda; double *A = qr_matrix(c, s, lda);
   const int st = nt / c.Nwrap;
   blk_copy(c.ULTd, N, c.ULTs + (size_t)st * NN, N, N, N);
@@ -15,21 +15,33 @@ __device__ __noinline__ void wrap_tau(const ChainDesc &c, const Smem &s, int nt,
   apply_pending_R(c, s, A, lda, pd.lo, pd.hi, c.use_kin != 0);
   pd.lo = 1; pd.hi = 0;
   chain_stab_U(c, s, A, lda, c.URd, c.DRd, c.VRd, false);
-  dev_stab_green_big(s, N, c.URd, c.DRd, c.VRd, c.ULTd, c.DLd, c.VLd, c.W0, c.W1, c.W2, c.W3,
-                     c.B0, c.B1, c.B2, c.B3);
-  const double *T = c.B3;
-  double d0 = blk_maxdiff(T + (size_t)N * n2, n2, c.G0t, N, N, s.red);
-  double d1 = blk_maxdiff(T + N, n2, c.Gt0, N, N, s.red);
-  double d2 = blk_maxdiff(T + N + (size_t)N * n2, n2, c.Gtt, N, N, s.red);
+  double *n00 = c.G00, *n0t = c.T0, *nt0 = c.T1, *ntt = c.T2;
+  dev_stab_green_big(s, N, c.URd, c.DRd, c.VRd, c.ULTd, c.DLd, c.VLd, A, lda, c.W0, c.W1, c.W2, c.W3,
+                     n00, n0t, nt0, ntt);
+  // the new blocks replace the propagated ones; their largest differences
+  double d0 = 0.0, d1 = 0.0, d2 = 0.0;
+  const auto swap_in = [&](double *dst, const double *src, double &d) {
+    blk_walk<8, double2>(
+        N, N, [&](int i, int j) { return make_double2(src[i + (size_t)j * N], dst[i + (size_t)j * N]); },
+        [&](double2 v, int i, int j) {
+          const double x = fabs(v.x - v.y);
+          d = (x > d || x != x) ? x : d;   // keep NaN visible
+          dst[i + (size_t)j * N] = v.x;
+        });
+    d = blk_max(d, s.red);
+    __syncthreads();
+  };
+  swap_in(c.G0t, n0t, d0);
+  swap_in(c.Gt0, nt0, d1);
+  swap_in(c.Gtt, ntt, d2);
   if (threadIdx.x == 0) {
     double d[3] = {d0, d1, d2};
     for (int q = 0; q < 3; ++q) {
       if (d[q] > c.acc[A_TXMAX0 + q] || d[q] != d[q]) c.acc[A_TXMAX0 + q] = d[q];
-      c.acc[A_TXMEAN0 + q] += d[q];
+      acc_add(c, A_TXMEAN0 + q, d[q]);
       if (!(d[q] == d[q]) || isinf(d[q])) atomicOr(c.status, ST_NONFINITE);
     }
   }
-  green_big_extract(N, T, c.G00, c.G0t, c.Gt0, c.Gtt);
 }
 
 // Dyn_reset (src/dynamics.f90:41-48, Propgr_reset src/process_matrix.f90:88-96):

@@ -97,19 +97,6 @@ __device__ __noinline__ void blk_scale_cols(double *A, int lda, int m, int n, co
   __syncthreads();
 }
 
-// max |A - B| (compare_mat, src/stabilization.f90:365-372)
-__device__ __noinline__ double blk_maxdiff(const double *A, int lda, const double *B, int ldb, int n, double *red) {
-  double m = 0.0;
-  for (int j = threadIdx.x / 32; j < n; j += Z2_WARPS)
-    for (int i = threadIdx.x & 31; i < n; i += 32) {
-      double d = fabs(A[i + (size_t)j * lda] - B[i + (size_t)j * ldb]);
-      m = (d > m || d != d) ? d : m;   // keep NaN visible
-    }
-  double r = blk_max(m, red);
-  __syncthreads();
-  return r;
-}
-
 // ---------------------------------------------------------------------------
 // Pivoted Householder QR (DGEQP3 -> DLAQP2 semantics, all columns free).
 // On exit A holds R and the reflectors, tau the scalar factors, jpvt the
@@ -136,7 +123,7 @@ __device__ __noinline__ void blk_geqp3(double *A, int lda, int n, int *jpvt, dou
       int oi = __shfl_xor_sync(Z2_FULL, bi, o);
       if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
     }
-    const int pvt = bi;
+    const int pvt = bi < n ? bi : j;   // no candidate: a column of NaNs
     __syncthreads();
     if (warp == 0) {
       double *Aj = A + (size_t)j * lda;
@@ -204,48 +191,6 @@ __device__ __noinline__ void blk_geqp3(double *A, int lda, int n, int *jpvt, dou
   }
 }
 
-// Unpivoted Householder QR (DGEQR2), used for the 2N x 2N UDV of the
-// time-displaced Green's function.
-__device__ __noinline__ void blk_geqr2(double *A, int lda, int m, int n, double *tau) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int kmax = m < n ? m : n;
-  for (int j = 0; j < kmax; ++j) {
-    if (warp == 0) {
-      double *Aj = A + (size_t)j * lda;
-      double s = 0.0;
-      for (int i = j + 1 + lane; i < m; i += 32) { double a = Aj[i]; s += a * a; }
-      s = warp_sum(s);
-      double alpha = Aj[j];
-      double t = 0.0, beta = alpha;
-      if (j < m - 1 && s != 0.0) {
-        double xnorm = sqrt(s);
-        beta = -copysign(dlapy2(alpha, xnorm), alpha);
-        t = (beta - alpha) / beta;
-        double sc = 1.0 / (alpha - beta);
-        for (int i = j + 1 + lane; i < m; i += 32) Aj[i] *= sc;
-      }
-      __syncwarp();
-      if (lane == 0) { tau[j] = t; Aj[j] = beta; }
-    }
-    __syncthreads();
-    const double tj = tau[j];
-    const double *v = A + (size_t)j * lda;
-    if (tj != 0.0) {
-      for (int k = j + 1 + warp; k < n; k += Z2_WARPS) {
-        double *Ak = A + (size_t)k * lda;
-        double w = 0.0;
-        for (int i = j + 1 + lane; i < m; i += 32) w += v[i] * Ak[i];
-        w = warp_sum(w) + Ak[j];
-        double tw = tj * w;
-        __syncwarp();
-        if (lane == 0) Ak[j] -= tw;
-        for (int i = j + 1 + lane; i < m; i += 32) Ak[i] -= v[i] * tw;
-      }
-    }
-    __syncthreads();
-  }
-}
-
 // QDRP_decompose's split (src/stabilization.f90:61-66): D(i) = |R(i,i)|,
 // R(i, i:n) /= D(i).
 // The rows are scaled by the reciprocal of D (one division per row instead
@@ -285,96 +230,4 @@ __device__ __noinline__ void blk_perm_cols(double *dst, int ldd, const double *s
     }
   }
   __syncthreads();
-}
-
-__device__ __forceinline__ double ld_op(const double *X, int ld, bool t, bool tri, int r, int c) {
-  // element (r, c) of op(X)
-  int sr = t ? c : r, sc = t ? r : c;
-  if (tri && sr > sc) return 0.0;
-  return X[sr + (size_t)sc * ld];
-}
-
-// ---------------------------------------------------------------------------
-// LU with partial pivoting and explicit inverse (stands in for LINPACK
-// ZGEFA/ZGEDI of INV_C, lib/package_of_matrix/Modules/mat_mod.f90:296-336).
-// A (n x n) is overwritten by its inverse; W is an n x n workspace.
-// ---------------------------------------------------------------------------
-__device__ __noinline__ void blk_inverse(double *A, int lda, int n, double *W, int ldw, int *ipiv,
-                            double *red, int *flag) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // LU (right-looking, unblocked)
-  for (int k = 0; k < n; ++k) {
-    double bv = -1.0; int bi = n;
-    for (int i = k + threadIdx.x; i < n; i += Z2_NT) {
-      double v = fabs(A[i + (size_t)k * lda]);
-      if (v > bv) { bv = v; bi = i; }
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      double ov = __shfl_xor_sync(Z2_FULL, bv, o);
-      int oi = __shfl_xor_sync(Z2_FULL, bi, o);
-      if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-    }
-    __syncthreads();
-    if (lane == 0) { red[warp] = bv; flag[warp] = bi; }
-    __syncthreads();
-    bv = red[0]; bi = flag[0];
-    for (int w = 1; w < Z2_WARPS; ++w)
-      if (red[w] > bv || (red[w] == bv && flag[w] < bi)) { bv = red[w]; bi = flag[w]; }
-    const int p = bi;
-    __syncthreads();
-    if (threadIdx.x == 0) ipiv[k] = p;
-    if (p != k)
-      for (int j = threadIdx.x; j < n; j += Z2_NT) {
-        double t = A[k + (size_t)j * lda];
-        A[k + (size_t)j * lda] = A[p + (size_t)j * lda];
-        A[p + (size_t)j * lda] = t;
-      }
-    __syncthreads();
-    const double piv = A[k + (size_t)k * lda];
-    for (int i = k + 1 + threadIdx.x; i < n; i += Z2_NT) A[i + (size_t)k * lda] /= piv;
-    __syncthreads();
-    for (int j = k + 1 + warp; j < n; j += Z2_WARPS) {
-      double akj = A[k + (size_t)j * lda];
-      if (akj != 0.0)
-        for (int i = k + 1 + lane; i < n; i += 32) A[i + (size_t)j * lda] -= A[i + (size_t)k * lda] * akj;
-    }
-    __syncthreads();
-  }
-  // inverse: solve L U X = P^T I column by column into W, then copy back
-  blk_identity(W, ldw, n);
-  // apply row interchanges to the identity
-  for (int c = threadIdx.x; c < n; c += Z2_NT)
-    for (int k = 0; k < n; ++k) {
-      int p = ipiv[k];
-      if (p != k) {
-        double t = W[k + (size_t)c * ldw];
-        W[k + (size_t)c * ldw] = W[p + (size_t)c * ldw];
-        W[p + (size_t)c * ldw] = t;
-      }
-    }
-  __syncthreads();
-  for (int c = warp; c < n; c += Z2_WARPS) {
-    double *Wc = W + (size_t)c * ldw;
-    // forward substitution with unit L
-    for (int k = 0; k < n; ++k) {
-      __syncwarp();
-      double bk = Wc[k];
-      if (bk != 0.0)
-        for (int i = k + 1 + lane; i < n; i += 32) Wc[i] -= bk * A[i + (size_t)k * lda];
-    }
-    // back substitution with U
-    for (int k = n - 1; k >= 0; --k) {
-      __syncwarp();
-      double bk = Wc[k];
-      if (bk != 0.0) {
-        bk = bk / A[k + (size_t)k * lda];
-        __syncwarp();
-        if (lane == 0) Wc[k] = bk;
-        for (int i = lane; i < k; i += 32) Wc[i] -= bk * A[i + (size_t)k * lda];
-      }
-    }
-  }
-  __syncthreads();
-  blk_copy(A, lda, W, ldw, n, n);
 }

@@ -307,11 +307,14 @@ __device__ __noinline__ void dev_stab_U_fast(const Smem &s, int N, double *A, in
 
 // M <- (M')^-1 of the scale-split middle matrix, up to a row order: with piv[j]
 // the pivot row of column j, M'^-1(j, piv[m]) = M(piv[j], m).  rRb, rLb, Rs, Ls
-// receive DRb^-1, DLb^-1, DRs, DLs (N doubles of shared memory each).
+// receive DRb^-1, DLb^-1, DRs, DLs (N doubles of shared memory each).  N a
+// multiple of 4; above the panel kernels' range the inverse comes from a
+// blocked LU through the N x N global workspaces W0, W1.
 __device__ __noinline__ void middle_inverse(const Smem &s, int N, const double *UR, const double *DR,
                                             const double *VR, const double *ULT, const double *DL,
                                             const double *VL, double *M, int ldm, double *rRb,
-                                            double *rLb, double *Rs, double *Ls, int *piv) {
+                                            double *rLb, double *Rs, double *Ls, int *piv, double *W0,
+                                            double *W1) {
   for (int i = threadIdx.x; i < N; i += Z2_NT) {
     rRb[i] = 1.0 / fmax(DR[i], 1.0);
     rLb[i] = 1.0 / fmax(DL[i], 1.0);
@@ -322,7 +325,13 @@ __device__ __noinline__ void middle_inverse(const Smem &s, int N, const double *
   gemm_nnn(N, MatRef{UR, N, 1}, nullptr, false, MatRef{ULT, 1, N}, false, GemmOut{M, ldm});
   gemm_nnn(N, MatRef{VR, 1, N}, nullptr, false, MatRef{VL, 1, N}, false,
            GemmOut{M, ldm, rRb, rLb, Rs, Ls});
-  gj_any(M, ldm, N, piv, s.tile);
+  if (wy_ok(N, s.tile_doubles)) {
+    gj_any(M, ldm, N, piv, s.tile);
+  } else {
+    blk_inverse_blocked(M, ldm, N, W0, N, piv, s.red, s.flag, s.tile);
+    for (int i = threadIdx.x; i < N; i += Z2_NT) piv[i] = i;
+    __syncthreads();
+  }
 }
 
 // stab_green with the scale-split middle matrix; arguments as dev_stab_green
@@ -339,7 +348,8 @@ __device__ __noinline__ void dev_stab_green_fast(const Smem &s, int N, int nt, i
   }
   double *rRb = s.vec + N, *rLb = s.vec + 2 * N;
   int *piv = s.ivec;
-  middle_inverse(s, N, UR, DR, VR, ULT, DL, VL, M, ldm, rRb, rLb, s.vec + 3 * N, s.vec + 4 * N, piv);
+  middle_inverse(s, N, UR, DR, VR, ULT, DL, VL, M, ldm, rRb, rLb, s.vec + 3 * N, s.vec + 4 * N, piv,
+                 W1, W2);
   // columns of M into M'^-1's order, times DRb^-1: W1 = DLb^-1 M'^-1 DRb^-1 UR^T,
   // G = UL^T W1
   int *inv = piv + N;
