@@ -15,7 +15,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 SRC = os.path.join(HERE, "csrc", "z2_api.cu")
 OUT = os.path.join(HERE, "libz2dqmc.so")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo",
-              "-std=c++17", "-shared", "-Xcompiler", "-fPIC"]
+              "-std=c++17", "-rdc=true", "-shared", "-Xcompiler", "-fPIC"]
 
 
 def nvcc() -> str:

@@ -16,7 +16,7 @@
 
 static_assert(PH_COUNT == Z2_NPHASE, "phase counters and the C ABI disagree");
 
-enum { OP_PRE = 1, OP_SWEEP = 2, OP_LOGDET = 3, OP_GLOBAL = 4, OP_THERM = 5 };
+enum { OP_PRE = 1, OP_SWEEP = 2, OP_LOGDET = 3, OP_GLOBAL = 4, OP_THERM = 5, OP_UNIT = 6, OP_STATE = 7 };
 enum { U_MMULT_R = 1, U_MMULT_L, U_STAB_UR, U_STAB_UL, U_STAB_GREEN, U_STAB_GREEN_BIG };
 
 struct UnitArgs {
@@ -25,6 +25,21 @@ struct UnitArgs {
   const double *UR, *DR, *VR, *ULT, *DL, *VL;
   double *G, *G0t, *Gt0, *Gtt;    // outputs
   int nt, nflag;
+};
+
+// Module procedures on a chain's resident state (OP_STATE).
+enum {
+  SO_PROPK_PRE = 1, SO_PROPT_PRE, SO_PROPK_L, SO_PROPK_R, SO_PROPT_L, SO_PROPT_R,
+  SO_PROPGRK_R, SO_PROPGRT_R, SO_WRAP_PRE, SO_WRAP_L, SO_WRAP_R, SO_WRAP_TAU,
+  SO_DYN_RESET, SO_SWEEP_RESET, SO_OBS_EQ_CALC, SO_OBS_EQ_AVE, SO_OBS_TAU_CALC,
+  SO_OBS_TAU_AVE, SO_SLICE_L, SO_SLICE_R
+};
+
+// Arguments of the module procedures.
+struct ModArgs {
+  UnitArgs u;
+  int nt, flag;
+  double x;
 };
 
 // ---------------------------------------------------------------------------
@@ -37,50 +52,8 @@ __device__ __forceinline__ void load_desc(ChainDesc &sc, const ChainDesc *g) {
   __syncthreads();
 }
 
-// Persistent launch: every CTA pulls chains from a work queue (ordered by
-// decreasing cost) and runs the whole operation of that chain.
-__global__ void __launch_bounds__(Z2_NT, 1)
-z2_chain_kernel(const ChainDesc *descs, const int *order, int nchains, int *queue, int op,
-                int nsweep, int toggle, unsigned smem_bytes) {
-  __shared__ ChainDesc sc;
-  __shared__ Smem s;     // pointer table in shared memory, not on the local stack
-  __shared__ int s_idx;
-  for (;;) {
-    if (threadIdx.x == 0) s_idx = atomicAdd(queue, 1);
-    __syncthreads();
-    const int idx = s_idx;
-    if (idx >= nchains) break;
-    load_desc(sc, descs + order[idx]);
-    if (threadIdx.x == 0) s = make_smem(sc, z2_smem, smem_bytes);
-    __syncthreads();
-    if (op == OP_PRE) {
-      for (int i = threadIdx.x; i < 2 * sc.nb; i += Z2_NT) s.bond[i] = sc.bonds[i];
-      __syncthreads();
-      chain_pre(sc, s);
-    } else if (op == OP_SWEEP) {
-      chain_sweep(sc, s, nsweep, toggle != 0, sc.hzero ? 1.0 : 0.0);
-    } else if (op == OP_LOGDET) {
-      chain_logdet_grad(sc, s);
-    } else if (op == OP_GLOBAL) {
-      chain_global(sc, s, nsweep);
-    } else if (op == OP_THERM) {
-      chain_therm(sc, s, nsweep);
-    }
-    __syncthreads();
-  }
-}
-
-__global__ void __launch_bounds__(Z2_NT, 1)
-z2_state_kernel(const ChainDesc *desc, int op, int nt, int flag, double x, unsigned smem_bytes);
-
-// Module-level mirrors on single matrices, one CTA.
-__global__ void __launch_bounds__(Z2_NT, 1)
-z2_unit_kernel(const ChainDesc *desc, int op, UnitArgs a, unsigned smem_bytes) {
-  __shared__ ChainDesc sc;
-  __shared__ Smem s;
-  load_desc(sc, desc);
-  if (threadIdx.x == 0) s = make_smem(sc, z2_smem, smem_bytes);
-  __syncthreads();
+// A module procedure on single matrices, one CTA.
+__device__ __noinline__ void unit_op(const ChainDesc &sc, const Smem &s, int op, const UnitArgs &a) {
   const int N = sc.N;
   if (op == U_MMULT_R || op == U_MMULT_L) {
     build_table(sc, s, a.nt);
@@ -98,6 +71,159 @@ z2_unit_kernel(const ChainDesc *desc, int op, UnitArgs a, unsigned smem_bytes) {
     int lda; double *A = qr_matrix(sc, s, lda);
     dev_stab_green_big(s, N, a.UR, a.DR, a.VR, a.ULT, a.DL, a.VL, A, lda, sc.W0, sc.W1, sc.W2, sc.W3,
                        a.G, a.G0t, a.Gt0, a.Gtt);
+  }
+}
+
+// A procedure of the reference's modules on a chain's resident state, one CTA.
+__device__ __noinline__ void state_op(const ChainDesc &c, const Smem &s, int op, int nt, int flag, double x) {
+  const int N = c.N;
+  Pend pd{1, 0};
+  switch (op) {
+    case SO_PROPK_PRE:      // propK_pre (src/multiply.f90:8-15) as Local_sweep_pre calls it
+      if (c.use_kin) { build_table(c, s, nt); kin_global(c, s, c.UR, 1, 0); }
+      break;
+    case SO_PROPT_PRE:      // propT_pre (src/multiply.f90:65-77)
+      blk_scale(c.UR, N, N, N, c.eP);
+      break;
+    case SO_PROPK_L:        // propK_L (src/multiply.f90:17-28): G B, B^-1 G, UL B
+      load_G(c, s);
+      build_table(c, s, nt);
+      kin_cols(c, s, s.G, s.ldg, N, 1);
+      kin_rows(c, s, s.G, s.ldg, N, -1);
+      spill_G(c, s);
+      kin_global(c, s, c.ULT, 1, 0);      // UL^T <- B UL^T (B symmetric)
+      break;
+    case SO_PROPK_R:        // propK_R (src/multiply.f90:30-41): B G, G B^-1, B UR
+      load_G(c, s);
+      build_table(c, s, nt);
+      kin_rows(c, s, s.G, s.ldg, N, 1);
+      kin_cols(c, s, s.G, s.ldg, N, -1);
+      spill_G(c, s);
+      kin_global(c, s, c.UR, 1, 0);
+      break;
+    case SO_PROPT_L:        // propT_L (src/multiply.f90:79-93)
+      blk_scale(c.G, N, N, N, c.eP);
+      blk_scale(c.G, N, N, N, c.eM);
+      blk_scale(c.ULT, N, N, N, c.eP);
+      break;
+    case SO_PROPT_R:        // propT_R (src/multiply.f90:95-108)
+      blk_scale(c.G, N, N, N, c.eP);
+      blk_scale(c.G, N, N, N, c.eM);
+      blk_scale(c.UR, N, N, N, c.eP);
+      break;
+    case SO_PROPGRK_R:      // propgrK_R (src/multiply.f90:43-63) on the Dyn copy
+      if (c.use_kin) {
+        propgr_R(c, s, nt, true, false);
+        kin_global(c, s, c.URd, 1, 0);
+      }
+      break;
+    case SO_PROPGRT_R:      // propgrT_R (src/multiply.f90:110-130)
+      propgr_R(c, s, nt, false, true);
+      blk_scale(c.URd, N, N, N, c.eP);
+      break;
+    case SO_WRAP_PRE:       // Wrap_pre (src/stabilization.f90:374-398)
+      wrap_pre(c, s, nt, pd);
+      break;
+    case SO_WRAP_L:         // Wrap_L (src/stabilization.f90:400-437)
+      load_G(c, s);
+      wrap_L(c, s, nt, pd, flag != 0);
+      spill_G(c, s);
+      break;
+    case SO_WRAP_R:         // Wrap_R (src/stabilization.f90:439-476)
+      load_G(c, s);
+      wrap_R(c, s, nt, pd, flag != 0);
+      spill_G(c, s);
+      break;
+    case SO_WRAP_TAU:       // Wrap_tau (src/stabilization.f90:478-514)
+      wrap_tau(c, s, nt, pd);
+      break;
+    case SO_DYN_RESET:      // Dyn_reset (src/dynamics.f90:41-48)
+      dyn_reset(c, s);
+      break;
+    case SO_SWEEP_RESET:    // Local_sweep_reset (src/local_sweep.f90:56-71)
+      sweep_reset(c, flag != 0, c.hzero != 0);
+      break;
+    case SO_OBS_EQ_CALC:    // Obs_equal%calc (src/obser_equal.f90:73-149)
+      load_G(c, s);
+      obs_equal(c, s, nt);
+      break;
+    case SO_OBS_EQ_AVE:     // Obs_equal%ave (src/obser_equal.f90:50-71)
+      obs_equal_ave(c, x);
+      break;
+    case SO_OBS_TAU_CALC:   // Obs_tau%calc (src/obser_tau.f90:56-133)
+      obs_tau(c, s, nt);
+      break;
+    case SO_OBS_TAU_AVE:    // Obs_tau%ave (src/obser_tau.f90:37-47)
+      obs_tau_ave(c, x);
+      break;
+    case SO_SLICE_L:        // LocalK_prop_L (src/localK.f90:347-373)
+    case SO_SLICE_R:        // LocalK_prop_R (src/localK.f90:375-398)
+      load_G(c, s);
+      if (op == SO_SLICE_L) {
+        propose_slice(c, s, nt, true, 0);            // bonds 2N..1
+        build_table(c, s, nt);
+        kin_cols(c, s, s.G, s.ldg, N, 1);
+        kin_rows(c, s, s.G, s.ldg, N, -1);
+        spill_G(c, s);
+        kin_global(c, s, c.ULT, 1, 0);
+      } else {
+        build_table(c, s, nt);
+        kin_rows(c, s, s.G, s.ldg, N, 1);
+        kin_cols(c, s, s.G, s.ldg, N, -1);
+        propose_slice(c, s, nt, false, 1);           // bonds 1..2N
+        spill_G(c, s);
+        build_table(c, s, nt);                       // B_nt with the flipped links
+        kin_global(c, s, c.UR, 1, 0);
+      }
+      break;
+    default:
+      break;
+  }
+}
+
+// Launch one state procedure on one chain, synchronously; a non-finite drift
+// or Green's function found by it is Z2_ERR_NONFINITE.
+
+// Persistent launch: every CTA pulls chains from a work queue (ordered by
+// decreasing cost) and runs the whole operation of that chain.  The module
+// procedures run in the same kernel (one CTA, queue null): one copy of the
+// device code instead of three.
+__global__ void __launch_bounds__(Z2_NT, 1)
+z2_chain_kernel(const ChainDesc *descs, const int *order, int nchains, int *queue, int op,
+                int nsweep, int toggle, unsigned smem_bytes, const __grid_constant__ ModArgs m) {
+  __shared__ ChainDesc sc;
+  __shared__ Smem s;     // pointer table in shared memory, not on the local stack
+  __shared__ int s_idx;
+  for (;;) {
+    if (queue != nullptr) {
+      if (threadIdx.x == 0) s_idx = atomicAdd(queue, 1);
+      __syncthreads();
+      const int idx = s_idx;
+      if (idx >= nchains) break;
+      load_desc(sc, descs + order[idx]);
+    } else {
+      load_desc(sc, descs);
+    }
+    if (threadIdx.x == 0) s = make_smem(sc, z2_smem, smem_bytes);
+    __syncthreads();
+    if (op != OP_THERM) kin_init(sc, s);
+    if (op == OP_PRE) {
+      chain_pre(sc, s);
+    } else if (op == OP_SWEEP) {
+      chain_sweep(sc, s, nsweep, toggle != 0, sc.hzero ? 1.0 : 0.0);
+    } else if (op == OP_LOGDET) {
+      chain_logdet_grad(sc, s);
+    } else if (op == OP_GLOBAL) {
+      chain_global(sc, s, nsweep);
+    } else if (op == OP_THERM) {
+      chain_therm(sc, s, nsweep);
+    } else if (op == OP_UNIT) {
+      unit_op(sc, s, nsweep, m.u);
+    } else if (op == OP_STATE) {
+      state_op(sc, s, nsweep, m.nt, m.flag, m.x);
+    }
+    if (queue == nullptr) break;
+    __syncthreads();
   }
 }
 
@@ -191,31 +317,31 @@ struct HostLattice {
   }
 };
 
-// L when the checkerboard table of an L x L lattice has the layout the fused
-// kinetic kernels assume (group 0/1: x bonds from odd/even x, slot
-// y L/2 + m; group 2/3: y bonds from odd/even y, slot m L + x; bond
-// orientation (site, next site)), else 0.
-int kin_fused_size(const HostLattice &lat) {
-  const int L = lat.Lx;
-  if (lat.Ly != L || L % 2 != 0 || L < 4 || L > 16 || !lat.ok) return 0;
-  const int H = L * L / 2, HL = L / 2;
+// Whether the checkerboard table has the layout of the line sweeps (group 0/1:
+// x bonds from odd/even x, slot y Lx/2 + m; group 2/3: y bonds from odd/even y,
+// slot m Lx + x; bond orientation (site, next site)) and both line lengths are
+// instantiated (even, 4 to 16).
+int kin_line_layout(const HostLattice &lat) {
+  const int Lx = lat.Lx, Ly = lat.Ly;
+  if (Lx % 2 || Ly % 2 || Lx < 4 || Ly < 4 || Lx > 16 || Ly > 16 || !lat.ok) return 0;
+  const int H = Lx * Ly / 2, HL = Lx / 2;
   auto check = [&](int g, int slot, int a, int b) {
     const int bd = lat.groups[g * H + slot];
     return lat.bonds[2 * bd] == a && lat.bonds[2 * bd + 1] == b;
   };
-  for (int y = 0; y < L; ++y)
+  for (int y = 0; y < Ly; ++y)
     for (int m = 0; m < HL; ++m) {
       const int xo = 2 * m + 1, xe = 2 * m;
-      if (!check(0, y * HL + m, y * L + xo, y * L + (xo + 1) % L)) return 0;
-      if (!check(1, y * HL + m, y * L + xe, y * L + xe + 1)) return 0;
+      if (!check(0, y * HL + m, y * Lx + xo, y * Lx + (xo + 1) % Lx)) return 0;
+      if (!check(1, y * HL + m, y * Lx + xe, y * Lx + xe + 1)) return 0;
     }
-  for (int m = 0; m < HL; ++m)
-    for (int x = 0; x < L; ++x) {
+  for (int m = 0; m < Ly / 2; ++m)
+    for (int x = 0; x < Lx; ++x) {
       const int yo = 2 * m + 1, ye = 2 * m;
-      if (!check(2, m * L + x, yo * L + x, ((yo + 1) % L) * L + x)) return 0;
-      if (!check(3, m * L + x, ye * L + x, (ye + 1) * L + x)) return 0;
+      if (!check(2, m * Lx + x, yo * Lx + x, ((yo + 1) % Ly) * Lx + x)) return 0;
+      if (!check(3, m * Lx + x, ye * Lx + x, (ye + 1) * Lx + x)) return 0;
     }
-  return L;
+  return 1;
 }
 
 struct ChainHost {
@@ -320,9 +446,9 @@ static size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 static int smem_small_bytes(int N) {
   size_t off = 0;
   auto a16 = [](size_t x) { return (x + 15) & ~size_t(15); };
-  off += 8 * Z2_NRED; off += 8 * 8 * N; off += 8 * 2 * N; off += 8 * 2 * N;
-  off += a16(4 * 2 * N); off += a16(4 * 4 * N); off += a16(4 * 4 * N); off += 4 * 16;
-  off += a16(6 * N);
+  off += 8 * Z2_NRED; off += 8 * 8 * N; off += 16 * 2 * N;
+  off += a16(4 * 2 * N); off += a16(4 * 4 * N); off += a16(4 * 4 * N); off += a16(2 * 2 * N);
+  off += 4 * 16; off += a16(2 * N);
   return (int)a16(off);
 }
 
@@ -364,13 +490,6 @@ extern "C" int z2_create(z2_handle **out, const z2_chain_params *params, int32_t
                      h->opt.flush_shape_chain[c], p.Nlx * p.Nly);
   }
   CUDA_TRY(h, cudaSetDevice(h->device));
-  // ranf multiplier powers
-  {
-    unsigned int pw[33];
-    uint64_t v = 1;
-    for (int i = 0; i <= 32; ++i) { pw[i] = (unsigned)v; v = (v * 48828125ull) & 0x7fffffffull; }
-    CUDA_TRY(h, cudaMemcpyToSymbol(c_ipow, pw, sizeof(pw)));
-  }
   h->ch.resize(nchains);
   int smem_needed = 0;
   for (int c = 0; c < nchains; ++c) {
@@ -438,10 +557,6 @@ extern "C" int z2_create(z2_handle **out, const z2_chain_params *params, int32_t
   }
   CUDA_TRY(h, cudaFuncSetAttribute(z2_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)h->smem));
-  CUDA_TRY(h, cudaFuncSetAttribute(z2_unit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)h->smem));
-  CUDA_TRY(h, cudaFuncSetAttribute(z2_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)h->smem));
   CUDA_TRY(h, cudaMalloc(&h->d_status, sizeof(int) * nchains));
   CUDA_TRY(h, cudaMemset(h->d_status, 0, sizeof(int) * nchains));
   h->h_status.assign(nchains, 0);
@@ -465,13 +580,16 @@ extern "C" int z2_create(z2_handle **out, const z2_chain_params *params, int32_t
       dlt[2 * b + 1] = s_new * c_old - c_new * s_old;
     }
     for (int s = 0; s < N; ++s) stag[s] = ((lat.xy[2 * s] + lat.xy[2 * s + 1]) % 2 == 0) ? 1.0 : -1.0;
-    const int W = 2 * p.Nlx - 1, H = 2 * p.Nly - 1;
-    std::vector<double> psh((size_t)W * H);
+    // site factors of the shifted cdw phase cos(qx dx + pi dy)
+    // (src/obser_equal.f90:98-149)
+    std::vector<double> phase(2 * (size_t)N);
     const double PI = std::acos(-1.0);
     const double qx = PI - 2.0 * PI / (double)p.Nlx;
-    for (int dy = -(p.Nly - 1); dy <= p.Nly - 1; ++dy)
-      for (int dx = -(p.Nlx - 1); dx <= p.Nlx - 1; ++dx)
-        psh[(dx + p.Nlx - 1) + (size_t)(dy + p.Nly - 1) * W] = std::cos(qx * (double)dx + PI * (double)dy);
+    for (int i = 0; i < N; ++i) {
+      const double sy = (lat.xy[2 * i + 1] % 2) ? -1.0 : 1.0;
+      phase[2 * i] = sy * std::cos(qx * (double)lat.xy[2 * i]);
+      phase[2 * i + 1] = sy * std::sin(qx * (double)lat.xy[2 * i]);
+    }
     // boson ratio table (src/fields.f90:52-117)
     double rb[9];
     {
@@ -505,7 +623,7 @@ extern "C" int z2_create(z2_handle **out, const z2_chain_params *params, int32_t
     size_t o_bb = take(4 * lat.bbonds.size()), o_plaq = take(4 * lat.plaq.size());
     size_t o_xy = take(4 * lat.xy.size()), o_nbx = take(4 * lat.nbx.size());
     size_t o_chsh = take(8 * chsh.size()), o_dlt = take(8 * dlt.size());
-    size_t o_stag = take(8 * stag.size()), o_psh = take(8 * psh.size());
+    size_t o_stag = take(8 * stag.size()), o_phase = take(8 * phase.size());
     size_t o_sigma = take((size_t)nb * Lt);
     size_t o_mat = take(8 * NN * 10);             // G, UR, VR, ULT, VL, W0..W4
     size_t o_vec = take(8 * (size_t)N * 2);       // DR, DL
@@ -540,7 +658,7 @@ extern "C" int z2_create(z2_handle **out, const z2_chain_params *params, int32_t
     CUDA_TRY(h, up(o_chsh, chsh.data(), 8 * chsh.size()));
     CUDA_TRY(h, up(o_dlt, dlt.data(), 8 * dlt.size()));
     CUDA_TRY(h, up(o_stag, stag.data(), 8 * stag.size()));
-    CUDA_TRY(h, up(o_psh, psh.data(), 8 * psh.size()));
+    CUDA_TRY(h, up(o_phase, phase.data(), 8 * phase.size()));
     CUDA_TRY(h, up(o_sigma, C.sigma0.data(), C.sigma0.size()));
     if (h->opt.tau) {
       // exp(i k.r) of Fourier_R_to_K (src/lattice.f90:159-173, 263-281):
@@ -579,12 +697,12 @@ extern "C" int z2_create(z2_handle **out, const z2_chain_params *params, int32_t
     d.hzero = std::fabs(p.h) <= kZero ? 1 : 0;
     d.stab_exact = h->opt.stab_exact ? 1 : 0;
     d.flush_shape = h->opt.flush_shape_chain ? h->opt.flush_shape_chain[c] : 0;
-    d.kin_fused = kin_fused_size(lat);
+    d.kin_lines = kin_line_layout(lat);
     d.bonds = (const int *)(base + o_bonds); d.groups = (const int *)(base + o_groups);
     d.bbonds = (const int *)(base + o_bb); d.plaq = (const int *)(base + o_plaq);
     d.xy = (const int *)(base + o_xy); d.nbx = (const int *)(base + o_nbx);
     d.chsh = (const double *)(base + o_chsh); d.dlt = (const double *)(base + o_dlt);
-    d.stag = (const double *)(base + o_stag); d.pshift = (const double *)(base + o_psh);
+    d.stag = (const double *)(base + o_stag); d.phase = (const double *)(base + o_phase);
     d.sigma = (signed char *)(base + o_sigma);
     double *m = (double *)(base + o_mat);
     d.G = m; d.UR = m + NN; d.VR = m + 2 * NN; d.ULT = m + 3 * NN; d.VL = m + 4 * NN;
@@ -732,7 +850,7 @@ extern "C" int z2_get_config(const z2_handle *h, int32_t chain, double *sigma, i
 static int enqueue_chains(z2_handle *h, int op, int nsweep, int toggle) {
   CUDA_TRY(h, cudaMemsetAsync(h->d_queue, 0, sizeof(int), h->stream));
   z2_chain_kernel<<<h->grid, Z2_NT, h->smem, h->stream>>>(h->d_desc, h->d_order, h->nchains,
-                                                          h->d_queue, op, nsweep, toggle, h->smem);
+                                                          h->d_queue, op, nsweep, toggle, h->smem, ModArgs{});
   CUDA_TRY(h, cudaGetLastError());
   return Z2_OK;
 }
@@ -1175,7 +1293,7 @@ extern "C" int z2_logdet_grad(z2_handle *h, int32_t chain, double *logdet, doubl
   CUDA_TRY(h, cudaMemcpy(d_one, &chain, sizeof(int), cudaMemcpyHostToDevice));
   CUDA_TRY(h, cudaMemsetAsync(h->d_queue, 0, sizeof(int), h->stream));
   z2_chain_kernel<<<1, Z2_NT, h->smem, h->stream>>>(h->d_desc, d_one, 1, h->d_queue, OP_LOGDET, 0,
-                                                     0, h->smem);
+                                                     0, h->smem, ModArgs{});
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   cudaFree(d_one);
@@ -1200,7 +1318,10 @@ static int unit_scratch(z2_handle *h, size_t doubles) {
 }
 
 static int run_unit(z2_handle *h, int chain, int op, const UnitArgs &a) {
-  z2_unit_kernel<<<1, Z2_NT, h->smem, h->stream>>>(h->d_desc + chain, op, a, h->smem);
+  ModArgs m{};
+  m.u = a;
+  z2_chain_kernel<<<1, Z2_NT, h->smem, h->stream>>>(h->d_desc + chain, nullptr, 1, nullptr, OP_UNIT, op, 0,
+                                                    h->smem, m);
   CUDA_TRY(h, cudaGetLastError());
   CUDA_TRY(h, cudaStreamSynchronize(h->stream));
   return Z2_OK;
@@ -1342,133 +1463,15 @@ extern "C" int z2_stab_green_big(z2_handle *h, int32_t chain, const double *UR, 
 // call (the whole-bin path propagates them lazily, with the same operations in
 // the same order).  One CTA, the chain kernel's shared-memory plan.
 // ---------------------------------------------------------------------------
-enum {
-  SO_PROPK_PRE = 1, SO_PROPT_PRE, SO_PROPK_L, SO_PROPK_R, SO_PROPT_L, SO_PROPT_R,
-  SO_PROPGRK_R, SO_PROPGRT_R, SO_WRAP_PRE, SO_WRAP_L, SO_WRAP_R, SO_WRAP_TAU,
-  SO_DYN_RESET, SO_SWEEP_RESET, SO_OBS_EQ_CALC, SO_OBS_EQ_AVE, SO_OBS_TAU_CALC,
-  SO_OBS_TAU_AVE, SO_SLICE_L, SO_SLICE_R
-};
 
-__global__ void __launch_bounds__(Z2_NT, 1)
-z2_state_kernel(const ChainDesc *desc, int op, int nt, int flag, double x, unsigned smem_bytes) {
-  __shared__ ChainDesc sc;
-  __shared__ Smem s;
-  load_desc(sc, desc);
-  if (threadIdx.x == 0) s = make_smem(sc, z2_smem, smem_bytes);
-  __syncthreads();
-  const ChainDesc &c = sc;
-  const int N = c.N;
-  Pend pd{1, 0};
-  switch (op) {
-    case SO_PROPK_PRE:      // propK_pre (src/multiply.f90:8-15) as Local_sweep_pre calls it
-      if (c.use_kin) { build_table(c, s, nt); kin_global(c, s, c.UR, 1, 0); }
-      break;
-    case SO_PROPT_PRE:      // propT_pre (src/multiply.f90:65-77)
-      blk_scale(c.UR, N, N, N, c.eP);
-      break;
-    case SO_PROPK_L:        // propK_L (src/multiply.f90:17-28): G B, B^-1 G, UL B
-      load_G(c, s);
-      build_table(c, s, nt);
-      kin_cols(c, s, s.G, s.ldg, N, 1);
-      kin_rows(c, s, s.G, s.ldg, N, -1);
-      spill_G(c, s);
-      kin_global(c, s, c.ULT, 1, 0);      // UL^T <- B UL^T (B symmetric)
-      break;
-    case SO_PROPK_R:        // propK_R (src/multiply.f90:30-41): B G, G B^-1, B UR
-      load_G(c, s);
-      build_table(c, s, nt);
-      kin_rows(c, s, s.G, s.ldg, N, 1);
-      kin_cols(c, s, s.G, s.ldg, N, -1);
-      spill_G(c, s);
-      kin_global(c, s, c.UR, 1, 0);
-      break;
-    case SO_PROPT_L:        // propT_L (src/multiply.f90:79-93)
-      blk_scale(c.G, N, N, N, c.eP);
-      blk_scale(c.G, N, N, N, c.eM);
-      blk_scale(c.ULT, N, N, N, c.eP);
-      break;
-    case SO_PROPT_R:        // propT_R (src/multiply.f90:95-108)
-      blk_scale(c.G, N, N, N, c.eP);
-      blk_scale(c.G, N, N, N, c.eM);
-      blk_scale(c.UR, N, N, N, c.eP);
-      break;
-    case SO_PROPGRK_R:      // propgrK_R (src/multiply.f90:43-63) on the Dyn copy
-      if (c.use_kin) {
-        propgr_R(c, s, nt, true, false);
-        kin_global(c, s, c.URd, 1, 0);
-      }
-      break;
-    case SO_PROPGRT_R:      // propgrT_R (src/multiply.f90:110-130)
-      propgr_R(c, s, nt, false, true);
-      blk_scale(c.URd, N, N, N, c.eP);
-      break;
-    case SO_WRAP_PRE:       // Wrap_pre (src/stabilization.f90:374-398)
-      wrap_pre(c, s, nt, pd);
-      break;
-    case SO_WRAP_L:         // Wrap_L (src/stabilization.f90:400-437)
-      load_G(c, s);
-      wrap_L(c, s, nt, pd, flag != 0);
-      spill_G(c, s);
-      break;
-    case SO_WRAP_R:         // Wrap_R (src/stabilization.f90:439-476)
-      load_G(c, s);
-      wrap_R(c, s, nt, pd, flag != 0);
-      spill_G(c, s);
-      break;
-    case SO_WRAP_TAU:       // Wrap_tau (src/stabilization.f90:478-514)
-      wrap_tau(c, s, nt, pd);
-      break;
-    case SO_DYN_RESET:      // Dyn_reset (src/dynamics.f90:41-48)
-      dyn_reset(c, s);
-      break;
-    case SO_SWEEP_RESET:    // Local_sweep_reset (src/local_sweep.f90:56-71)
-      sweep_reset(c, flag != 0, c.hzero != 0);
-      break;
-    case SO_OBS_EQ_CALC:    // Obs_equal%calc (src/obser_equal.f90:73-149)
-      load_G(c, s);
-      obs_equal(c, s, nt);
-      break;
-    case SO_OBS_EQ_AVE:     // Obs_equal%ave (src/obser_equal.f90:50-71)
-      obs_equal_ave(c, x);
-      break;
-    case SO_OBS_TAU_CALC:   // Obs_tau%calc (src/obser_tau.f90:56-133)
-      obs_tau(c, s, nt);
-      break;
-    case SO_OBS_TAU_AVE:    // Obs_tau%ave (src/obser_tau.f90:37-47)
-      obs_tau_ave(c, x);
-      break;
-    case SO_SLICE_L:        // LocalK_prop_L (src/localK.f90:347-373)
-    case SO_SLICE_R:        // LocalK_prop_R (src/localK.f90:375-398)
-      for (int i = threadIdx.x; i < 2 * c.nb; i += Z2_NT) s.bond[i] = c.bonds[i];
-      __syncthreads();
-      load_G(c, s);
-      if (op == SO_SLICE_L) {
-        propose_slice(c, s, nt, true, 0);            // bonds 2N..1
-        build_table(c, s, nt);
-        kin_cols(c, s, s.G, s.ldg, N, 1);
-        kin_rows(c, s, s.G, s.ldg, N, -1);
-        spill_G(c, s);
-        kin_global(c, s, c.ULT, 1, 0);
-      } else {
-        build_table(c, s, nt);
-        kin_rows(c, s, s.G, s.ldg, N, 1);
-        kin_cols(c, s, s.G, s.ldg, N, -1);
-        propose_slice(c, s, nt, false, 1);           // bonds 1..2N
-        spill_G(c, s);
-        build_table(c, s, nt);                       // B_nt with the flipped links
-        kin_global(c, s, c.UR, 1, 0);
-      }
-      break;
-    default:
-      break;
-  }
-}
-
-// Launch one state procedure on one chain, synchronously; a non-finite drift
-// or Green's function found by it is Z2_ERR_NONFINITE.
 static int run_state(z2_handle *h, int chain, int op, int nt, int flag, double x) {
   CUDA_TRY(h, cudaSetDevice(h->device));
-  z2_state_kernel<<<1, Z2_NT, h->smem, h->stream>>>(h->d_desc + chain, op, nt, flag, x, h->smem);
+  ModArgs m{};
+  m.nt = nt;
+  m.flag = flag;
+  m.x = x;
+  z2_chain_kernel<<<1, Z2_NT, h->smem, h->stream>>>(h->d_desc + chain, nullptr, 1, nullptr, OP_STATE, op, 0,
+                                                    h->smem, m);
   CUDA_TRY(h, cudaGetLastError());
   CUDA_TRY(h, cudaStreamSynchronize(h->stream));
   int st = 0;

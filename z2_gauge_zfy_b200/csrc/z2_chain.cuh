@@ -9,11 +9,9 @@
 // update, and the U factors of the UDV chains are propagated lazily (all
 // Nwrap slices at once, right before the stabilization that needs them).
 #pragma once
+#include "z2_kin.cuh"
 #include "z2_propose.cuh"
 #include "z2_stab.cuh"
-
-// Checkerboard group order of one B (src/operator_kin.f90:74-85).
-__device__ __constant__ int c_gorder[8] = {0, 1, 2, 3, 3, 2, 1, 0};
 
 // ---------------------------------------------------------------------------
 // Shared-memory layout
@@ -26,13 +24,13 @@ __device__ Smem make_smem(const ChainDesc &c, unsigned char *base, size_t smem_b
   size_t off = 0;
   s.red = (double *)(base + off); off += sizeof(double) * Z2_NRED;
   s.vec = (double *)(base + off); off += sizeof(double) * 8 * N;
-  s.tc = (double *)(base + off); off += sizeof(double) * 2 * N;
-  s.ts = (double *)(base + off); off += sizeof(double) * 2 * N;
+  s.cs = (double2 *)(base + off); off += sizeof(double2) * 2 * N;
   s.ivec = (int *)(base + off); off += align16(sizeof(int) * 2 * N);
   s.tp = (int *)(base + off); off += align16(sizeof(int) * 4 * N);
   s.bond = (int *)(base + off); off += align16(sizeof(int) * 4 * N);
+  s.gid = (short *)(base + off); off += align16(sizeof(short) * 2 * N);
   s.flag = (int *)(base + off); off += sizeof(int) * 16;
-  s.sig = (signed char *)(base + off); off += align16(6 * N);   // slices nt, nt-1, nt+1
+  s.sig = (signed char *)(base + off); off += align16(2 * N);
   off = align16(off);
   s.arena = (double *)(base + off);
   const size_t arena_doubles = (smem_bytes - off) / sizeof(double);
@@ -54,369 +52,28 @@ __device__ Smem make_smem(const ChainDesc &c, unsigned char *base, size_t smem_b
   return s;
 }
 
-// ---------------------------------------------------------------------------
-// Checkerboard kinetic propagator (src/operator_kin.f90:61-179)
-// ---------------------------------------------------------------------------
-// Slice table in group order: position q = g*half + k holds bond groups[q].
-__device__ __noinline__ void build_table(const ChainDesc &c, const Smem &s, int nt) {
-  const signed char *sg = c.sigma + (size_t)(nt - 1) * c.nb;
-  for (int q = threadIdx.x; q < c.nb; q += Z2_NT) {
-    int b = c.groups[q];
-    s.tp[2 * q] = c.bonds[2 * b];
-    s.tp[2 * q + 1] = c.bonds[2 * b + 1];
-    s.tc[q] = c.chsh[2 * b];
-    s.ts[q] = (double)sg[b] * c.chsh[2 * b + 1];   // sinh(alpha*sigma) = sigma*sinh(alpha)
-  }
-  __syncthreads();
-}
-
-// One bond of a checkerboard group (process_group): [a, b] <- [[C, S], [S, C]]
-// [a, b], with the rounding sequence fixed (one product, one FMA per output)
-// so that every kinetic kernel below gives the same bits.
-__device__ __forceinline__ void kin_rot(double &a, double &b, double C, double S) {
-  const double na = __fma_rn(C, a, __dmul_rn(S, b));
-  const double nb = __fma_rn(S, a, __dmul_rn(C, b));
-  a = na;
-  b = nb;
-}
-
-// M <- B^nflag M : rows P1, P2 rotated by [[C,S],[S,C]] (process_group).
-// Row rotations never mix columns, so one thread carries its column through
-// all eight group passes: no barrier between passes.
-// Bonds of one group are disjoint, so a batch of 8 rotations is loaded,
-// rotated and stored as a whole (no store-to-load ordering inside a batch).
-template <bool ROWS>
-__device__ __forceinline__ void kin_group_vec(const Smem &s, double *base, size_t stride, int g0,
-                                              int half, double fl) {
-  // table pointers in registers (the Smem struct would otherwise be re-read
-  // after every store, which may alias it)
-  const int2 *__restrict__ tp2 = reinterpret_cast<const int2 *>(s.tp);
-  const double *__restrict__ tc = s.tc;
-  const double *__restrict__ ts = s.ts;
-  int kq = 0;
-  for (; kq + 7 < half; kq += 8) {
-    int2 pp[8];
-    double C[8], S[8], a[8], b[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      pp[q] = tp2[g0 + kq + q];
-      C[q] = tc[g0 + kq + q];
-      S[q] = fl * ts[g0 + kq + q];
-    }
-#pragma unroll
-    for (int q = 0; q < 8; ++q) { a[q] = base[pp[q].x * stride]; b[q] = base[pp[q].y * stride]; }
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      kin_rot(a[q], b[q], C[q], S[q]);
-      base[pp[q].x * stride] = a[q];
-      base[pp[q].y * stride] = b[q];
-    }
-  }
-  for (; kq < half; ++kq) {
-    const int2 pp = tp2[g0 + kq];
-    const double C = tc[g0 + kq], S = fl * ts[g0 + kq];
-    double a = base[pp.x * stride], b = base[pp.y * stride];
-    kin_rot(a, b, C, S);
-    base[pp.x * stride] = a;
-    base[pp.y * stride] = b;
-  }
-}
-
-// Fused passes on an L x L lattice with periodic boundaries (sites
-// y L + x).  The four groups are the x bonds from odd x (group 0) and from
-// even x (group 1), and the y bonds from odd y (group 2) and from even y
-// (group 3), each listed row by row (HostLattice, src/lattice.f90:72-102):
-//   group 0: bond (y L + x, y L + x+1 mod L), x = 2m+1, table slot y L/2 + m
-//   group 1: x = 2m, same slots;  group 2: (y L + x, (y+1 mod L) L + x),
-//   y = 2m+1, slot m L + x;  group 3: y = 2m, same slots.
-// Groups 0 and 1 only mix the sites of one lattice row and groups 2 and 3
-// only those of one lattice column, so the pass sequence 0 1 | 2 3 3 2 | 1 0
-// runs as three sweeps over lines: a thread loads one line of one matrix
-// column (or row) into registers, applies its passes and stores it, instead
-// of streaming the whole matrix through shared memory once per pass.  The
-// rotations and their order within each bond are those of the pass-by-pass
-// kernel, so the results are bitwise equal.
-template <int L>
-__device__ __forceinline__ void kin_line_odd(double (&v)[L], const double *__restrict__ tc,
-                                             const double *__restrict__ ts, double fl, int q0,
-                                             int qs) {
-#pragma unroll
-  for (int m = 0; m < L / 2; ++m) {
-    const int q = q0 + m * qs;
-    kin_rot(v[2 * m + 1], v[(2 * m + 2) % L], tc[q], fl * ts[q]);
-  }
-}
-template <int L>
-__device__ __forceinline__ void kin_line_even(double (&v)[L], const double *__restrict__ tc,
-                                              const double *__restrict__ ts, double fl, int q0,
-                                              int qs) {
-#pragma unroll
-  for (int m = 0; m < L / 2; ++m) {
-    const int q = q0 + m * qs;
-    kin_rot(v[2 * m], v[2 * m + 1], tc[q], fl * ts[q]);
-  }
-}
-
-// The three sweeps for n independent vectors: vector i's site k sits at
-// M[i * vs + k * ks] (kin_rows: vs = ld, ks = 1; kin_cols: vs = 1, ks = ld).
-// Threads take (vector, line) pairs, vector fastest, so a warp touches one
-// line of 32 consecutive vectors.
-template <int L>
-__device__ __noinline__ void kin_fused(const Smem &s, double *M, size_t vs, size_t ks, int n,
-                                       int nflag) {
-  constexpr int H = L * L / 2, HL = L / 2;
-  const double fl = (double)nflag;
-  const double *__restrict__ tc = s.tc;
-  const double *__restrict__ ts = s.ts;
-  const int tasks = n * L;
-  // a lattice row of one matrix column is contiguous when ks == 1: with an
-  // even column stride and an aligned matrix it moves as 16-byte pairs
-  const bool pairs = ks == 1 && (vs & 1) == 0 && (reinterpret_cast<size_t>(M) & 15) == 0;
-  // groups 0, 1 on lattice rows
-  for (int t = threadIdx.x; t < tasks; t += Z2_NT) {
-    const int i = t % n, y = t / n;
-    double *p = M + (size_t)i * vs + (size_t)(y * L) * ks;
-    double v[L];
-    if (pairs) {
-#pragma unroll
-      for (int x = 0; x < L; x += 2) {
-        const double2 w = reinterpret_cast<const double2 *>(p)[x >> 1];
-        v[x] = w.x; v[x + 1] = w.y;
-      }
-    } else {
-#pragma unroll
-      for (int x = 0; x < L; ++x) v[x] = p[(size_t)x * ks];
-    }
-    kin_line_odd<L>(v, tc, ts, fl, y * HL, 1);
-    kin_line_even<L>(v, tc, ts, fl, H + y * HL, 1);
-    if (pairs) {
-#pragma unroll
-      for (int x = 0; x < L; x += 2) reinterpret_cast<double2 *>(p)[x >> 1] = make_double2(v[x], v[x + 1]);
-    } else {
-#pragma unroll
-      for (int x = 0; x < L; ++x) p[(size_t)x * ks] = v[x];
-    }
-  }
-  __syncthreads();
-  // groups 2, 3, 3, 2 on lattice columns
-  for (int t = threadIdx.x; t < tasks; t += Z2_NT) {
-    const int i = t % n, x = t / n;
-    double *p = M + (size_t)i * vs + (size_t)x * ks;
-    double v[L];
-#pragma unroll
-    for (int y = 0; y < L; ++y) v[y] = p[(size_t)(y * L) * ks];
-    kin_line_odd<L>(v, tc, ts, fl, 2 * H + x, L);
-    kin_line_even<L>(v, tc, ts, fl, 3 * H + x, L);
-    kin_line_even<L>(v, tc, ts, fl, 3 * H + x, L);
-    kin_line_odd<L>(v, tc, ts, fl, 2 * H + x, L);
-#pragma unroll
-    for (int y = 0; y < L; ++y) p[(size_t)(y * L) * ks] = v[y];
-  }
-  __syncthreads();
-  // groups 1, 0 on lattice rows
-  for (int t = threadIdx.x; t < tasks; t += Z2_NT) {
-    const int i = t % n, y = t / n;
-    double *p = M + (size_t)i * vs + (size_t)(y * L) * ks;
-    double v[L];
-    if (pairs) {
-#pragma unroll
-      for (int x = 0; x < L; x += 2) {
-        const double2 w = reinterpret_cast<const double2 *>(p)[x >> 1];
-        v[x] = w.x; v[x + 1] = w.y;
-      }
-    } else {
-#pragma unroll
-      for (int x = 0; x < L; ++x) v[x] = p[(size_t)x * ks];
-    }
-    kin_line_even<L>(v, tc, ts, fl, H + y * HL, 1);
-    kin_line_odd<L>(v, tc, ts, fl, y * HL, 1);
-    if (pairs) {
-#pragma unroll
-      for (int x = 0; x < L; x += 2) reinterpret_cast<double2 *>(p)[x >> 1] = make_double2(v[x], v[x + 1]);
-    } else {
-#pragma unroll
-      for (int x = 0; x < L; ++x) p[(size_t)x * ks] = v[x];
-    }
-  }
-  __syncthreads();
-}
-
-// kin_fused for M <- M B (vectors are the rows of M, sites stride ld) when ld
-// is even: a thread takes two adjacent rows, so every site moves as one
-// 16-byte pair; the rotations and their order are kin_fused's.
-template <int L>
-__device__ __forceinline__ void kin_pair_odd(double (&v)[L], double (&w)[L], const double *__restrict__ tc,
-                                             const double *__restrict__ ts, double fl, int q0, int qs) {
-#pragma unroll
-  for (int m = 0; m < L / 2; ++m) {
-    const int q = q0 + m * qs;
-    const double C = tc[q], S = fl * ts[q];
-    kin_rot(v[2 * m + 1], v[(2 * m + 2) % L], C, S);
-    kin_rot(w[2 * m + 1], w[(2 * m + 2) % L], C, S);
-  }
-}
-template <int L>
-__device__ __forceinline__ void kin_pair_even(double (&v)[L], double (&w)[L], const double *__restrict__ tc,
-                                              const double *__restrict__ ts, double fl, int q0, int qs) {
-#pragma unroll
-  for (int m = 0; m < L / 2; ++m) {
-    const int q = q0 + m * qs;
-    const double C = tc[q], S = fl * ts[q];
-    kin_rot(v[2 * m], v[2 * m + 1], C, S);
-    kin_rot(w[2 * m], w[2 * m + 1], C, S);
-  }
-}
-template <int L>
-__device__ __noinline__ void kin_fused_rowpairs(const Smem &s, double *M, size_t ld, int n, int nflag) {
-  constexpr int H = L * L / 2, HL = L / 2;
-  const double fl = (double)nflag;
-  const double *__restrict__ tc = s.tc;
-  const double *__restrict__ ts = s.ts;
-  const int n2 = n >> 1, tasks = n2 * L;
-  for (int sweep = 0; sweep < 3; ++sweep) {
-    for (int t = threadIdx.x; t < tasks; t += Z2_NT) {
-      const int i = 2 * (t % n2), line = t / n2;
-      double v[L], w[L];
-      // sweep 0 and 2: lattice row `line` (sites line L + x); sweep 1:
-      // lattice column `line` (sites y L + line)
-      const size_t base = (sweep == 1) ? (size_t)line * ld : (size_t)(line * L) * ld;
-      const size_t step = (sweep == 1) ? (size_t)L * ld : ld;
-      double2 *p = reinterpret_cast<double2 *>(M + i + base);
-      const size_t st2 = step >> 1;
-#pragma unroll
-      for (int x = 0; x < L; ++x) {
-        const double2 u = p[(size_t)x * st2];
-        v[x] = u.x; w[x] = u.y;
-      }
-      if (sweep == 0) {
-        kin_pair_odd<L>(v, w, tc, ts, fl, line * HL, 1);
-        kin_pair_even<L>(v, w, tc, ts, fl, H + line * HL, 1);
-      } else if (sweep == 1) {
-        kin_pair_odd<L>(v, w, tc, ts, fl, 2 * H + line, L);
-        kin_pair_even<L>(v, w, tc, ts, fl, 3 * H + line, L);
-        kin_pair_even<L>(v, w, tc, ts, fl, 3 * H + line, L);
-        kin_pair_odd<L>(v, w, tc, ts, fl, 2 * H + line, L);
-      } else {
-        kin_pair_even<L>(v, w, tc, ts, fl, H + line * HL, 1);
-        kin_pair_odd<L>(v, w, tc, ts, fl, line * HL, 1);
-      }
-#pragma unroll
-      for (int x = 0; x < L; ++x) p[(size_t)x * st2] = make_double2(v[x], w[x]);
-    }
-    __syncthreads();
-  }
-}
-
-// kin_fused for the lattice sizes it is instantiated for; false otherwise.
-__device__ __forceinline__ bool kin_fused_any(int L, const Smem &s, double *M, size_t vs, size_t ks,
-                                              int n, int nflag) {
-  switch (L) {
-    case 4: kin_fused<4>(s, M, vs, ks, n, nflag); return true;
-    case 6: kin_fused<6>(s, M, vs, ks, n, nflag); return true;
-    case 8: kin_fused<8>(s, M, vs, ks, n, nflag); return true;
-    case 10: kin_fused<10>(s, M, vs, ks, n, nflag); return true;
-    case 12: kin_fused<12>(s, M, vs, ks, n, nflag); return true;
-    case 14: kin_fused<14>(s, M, vs, ks, n, nflag); return true;
-    case 16: kin_fused<16>(s, M, vs, ks, n, nflag); return true;
-    default: return false;
-  }
-}
-
-__device__ __noinline__ void kin_rows(const ChainDesc &c, const Smem &s, double *M, int ld, int ncols,
-                         int nflag) {
-  if (kin_fused_any(c.kin_fused, s, M, (size_t)ld, 1, ncols, nflag)) return;
-  const int half = c.half;
-  const double fl = (double)nflag;
-  for (int col = threadIdx.x; col < ncols; col += Z2_NT) {
-    double *mc = M + (size_t)col * ld;
-    for (int p = 0; p < 8; ++p) kin_group_vec<true>(s, mc, 1, c_gorder[p] * half, half, fl);
-  }
-  __syncthreads();
-}
-
-// M <- M B^nflag : columns P1, P2 rotated (process_group_L); one thread per
-// row through all eight passes.
-__device__ __noinline__ void kin_cols(const ChainDesc &c, const Smem &s, double *M, int ld, int nrows,
-                         int nflag) {
-  if ((ld & 1) == 0 && (nrows & 1) == 0 && (reinterpret_cast<size_t>(M) & 15) == 0) {
-    switch (c.kin_fused) {
-      case 4: kin_fused_rowpairs<4>(s, M, (size_t)ld, nrows, nflag); return;
-      case 6: kin_fused_rowpairs<6>(s, M, (size_t)ld, nrows, nflag); return;
-      case 8: kin_fused_rowpairs<8>(s, M, (size_t)ld, nrows, nflag); return;
-      case 10: kin_fused_rowpairs<10>(s, M, (size_t)ld, nrows, nflag); return;
-      case 12: kin_fused_rowpairs<12>(s, M, (size_t)ld, nrows, nflag); return;
-      case 14: kin_fused_rowpairs<14>(s, M, (size_t)ld, nrows, nflag); return;
-      case 16: kin_fused_rowpairs<16>(s, M, (size_t)ld, nrows, nflag); return;
-      default: break;
-    }
-  }
-  if (kin_fused_any(c.kin_fused, s, M, 1, (size_t)ld, nrows, nflag)) return;
-  const int half = c.half;
-  const double fl = (double)nflag;
-  for (int row = threadIdx.x; row < nrows; row += Z2_NT) {
-    double *mr = M + row;
-    for (int p = 0; p < 8; ++p) kin_group_vec<false>(s, mr, (size_t)ld, c_gorder[p] * half, half, fl);
-  }
-  __syncthreads();
-}
-
-// One group (one factor E_g) of B applied to rows / columns.
-__device__ __noinline__ void kin_group_rows(const ChainDesc &c, const Smem &s, double *M, int ld, int ncols,
-                               int g, int nflag) {
-  const int half = c.half, g0 = g * half;
-  const double fl = (double)nflag;
-  for (int col = threadIdx.x; col < ncols; col += Z2_NT)
-    kin_group_vec<true>(s, M + (size_t)col * ld, 1, g0, half, fl);
-  __syncthreads();
-}
-__device__ __noinline__ void kin_group_cols(const ChainDesc &c, const Smem &s, double *M, int ld, int nrows,
-                               int g, int nflag) {
-  const int half = c.half, g0 = g * half;
-  const double fl = (double)nflag;
-  for (int row = threadIdx.x; row < nrows; row += Z2_NT)
-    kin_group_vec<false>(s, M + row, (size_t)ld, g0, half, fl);
-  __syncthreads();
-}
-
-// Apply B-multiplications to a global N x N matrix, staging it through the
-// arena when it fits (the arena must be free).
-__device__ __noinline__ void kin_global(const ChainDesc &c, const Smem &s, double *M, int row_flag,
-                           int col_flag) {
-  const int N = c.N;
-  if (c.g_in_smem) {
-    double *A = s.arena;
-    blk_copy(A, c.ldg, M, N, N, N);
-    if (row_flag) kin_rows(c, s, A, c.ldg, N, row_flag);
-    if (col_flag) kin_cols(c, s, A, c.ldg, N, col_flag);
-    blk_copy(M, N, A, c.ldg, N, N);
-  } else {
-    if (row_flag) kin_rows(c, s, M, N, N, row_flag);
-    if (col_flag) kin_cols(c, s, M, N, N, col_flag);
-  }
-}
-
 // Lazily propagated U factors.  R chain: for nt' = lo..hi, U <- B_nt' U then
 // U *= e^{dtau mu} (LocalK_prop_R + propT_R, src/localK.f90:395-396,
 // src/multiply.f90:106).  L chain (ULT = UL^T, B symmetric): for nt' = hi
 // down to lo, ULT *= e^{dtau mu} then ULT <- B_nt' ULT (propT_L + prop_L,
 // src/multiply.f90:91, src/localK.f90:370).
-__device__ __noinline__ void apply_pending_R(const ChainDesc &c, const Smem &s, double *A, int lda, int lo,
-                                int hi, bool kin) {
-  for (int t = lo; t <= hi; ++t) {
-    if (kin) {
-      build_table(c, s, t);
-      kin_rows(c, s, A, lda, c.N, 1);
-    }
-    if (c.eP != 1.0) blk_scale(A, lda, c.N, c.N, c.eP);
-  }
+__device__ __noinline__ void pending_mu(const ChainDesc &c, double *A, int lda, int n) {
+  if (c.eP == 1.0) return;
+  double x = 1.0;
+  for (int i = 0; i < n; ++i) x *= c.eP;       // one pass for the n slices' factors
+  blk_scale(A, lda, c.N, c.N, x);
 }
-__device__ __noinline__ void apply_pending_L(const ChainDesc &c, const Smem &s, double *A, int lda, int lo,
+__device__ __forceinline__ void apply_pending_R(const ChainDesc &c, const Smem &s, double *A, int lda, int lo,
+                                int hi, bool kin) {
+  if (lo > hi) return;
+  if (kin) kin_slices(c, s, A, lda, lo, hi, 1, 1, 0);
+  pending_mu(c, A, lda, hi - lo + 1);
+}
+__device__ __forceinline__ void apply_pending_L(const ChainDesc &c, const Smem &s, double *A, int lda, int lo,
                                 int hi) {
-  for (int t = hi; t >= lo; --t) {
-    if (c.eP != 1.0) blk_scale(A, lda, c.N, c.N, c.eP);
-    build_table(c, s, t);
-    kin_rows(c, s, A, lda, c.N, 1);
-  }
+  if (lo > hi) return;
+  pending_mu(c, A, lda, hi - lo + 1);
+  kin_slices(c, s, A, lda, hi, lo, -1, 1, 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -473,61 +130,80 @@ __device__ __noinline__ void dev_stab_green_big(const Smem &s, int N, const doub
 // ---------------------------------------------------------------------------
 // Equal-time observables (Obs_equal_calc, src/obser_equal.f90:73-149)
 // ---------------------------------------------------------------------------
-__device__ __noinline__ void obs_equal(const ChainDesc &c, const Smem &s, int nt) {
-  const int N = c.N;
-  const double *G = s.G; const int ldg = s.ldg;
+//
+// With n_i = 1 - G_ii, t_ij = G_ij G_ji and the phases st_i st_j and
+// cos(qx dx + pi dy) = pc_i pc_j + ps_i ps_j (products of site factors), the
+// double sums split into squares of single sums and sums over unordered pairs:
+//   sum_ij ph_ij (4 n_i n_j - 2 (d_ij - G_ji) G_ij)
+//     = 4 (sum_i st_i n_i)^2 + 4 sum_{i<j} ph_ij t_ij - 2 sum_i (1 - G_ii) G_ii.
+// Pairs are taken along the diagonals (i, i + d mod N), d = 1..N/2 (d = N/2
+// meets each pair twice): lanes over i read G_ij and G_ji at the odd stride
+// ldg + 1, free of bank conflicts, and each warp has its share of the d.  (One
+// pass over all (i, j) with a gather of the phase took 20 K cycles per slice at
+// N = 144.)
+template <bool GS>
+__device__ __noinline__ void obs_equal_on(const ChainDesc &c, const Smem &s, int nt) {
+  const int N = c.N, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const double *G = GS ? as_shared(s.G) : s.G;
+  const int ldg = s.ldg;
   const signed char *sg = c.sigma + (size_t)(nt - 1) * c.nb;
-  double v[5] = {0, 0, 0, 0, 0};   // flux, pair, cdw, cdw_shift, density
-  for (int i = threadIdx.x; i < N; i += Z2_NT) {
-    const int *pl = c.plaq + 4 * i;
-    v[0] += (double)sg[pl[0]] * (double)sg[pl[1]] * (double)sg[pl[2]] * (double)sg[pl[3]];
-    double n = 1.0 - G[i + (size_t)i * ldg];
-    v[4] += n + n;
+  double *st = as_shared(s.vec), *pc = st + N, *ps = pc + N;
+  // flux, density, pairs, sums of st n, pc n, ps n, and the two pair sums
+  double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  for (int i = tid; i < N; i += Z2_NT) {
+    const int4 pl = reinterpret_cast<const int4 *>(c.plaq)[i];
+    const double a = c.stag[i], x = c.phase[2 * i], y = c.phase[2 * i + 1];
+    v[0] += (double)((int)sg[pl.x] * (int)sg[pl.y] * (int)sg[pl.z] * (int)sg[pl.w]);
+    const double g = G[i + (size_t)i * ldg], n = 1.0 - g;
+    st[i] = a;
+    pc[i] = x;
+    ps[i] = y;
+    v[1] += n + n;
+    v[2] += n * n;
+    v[3] += a * n;
+    v[4] += x * n;
+    v[5] += y * n;
+    v[6] -= 2.0 * n * g;
+    v[7] -= 2.0 * n * g;
   }
-  const int W = 2 * c.Lx - 1;
-  // task = (row i, one third of the columns j): the row's density, phase
-  // and coordinates stay in registers, the warp's lanes take consecutive
-  // rows (G(i, j) contiguous, G(j, i) at the stride ldg, column values
-  // broadcast), and no element needs an index division
-  const int J3 = (N + 2) / 3;
-  for (int t = threadIdx.x; t < 3 * N; t += Z2_NT) {
-    const int i = t % N, j0 = (t / N) * J3;
-    const int j1 = (j0 + J3 < N) ? j0 + J3 : N;
-    const double ni = 1.0 - G[i + (size_t)i * ldg];
-    const double sti = c.stag[i];
-    const int xi = c.xy[2 * i] + c.Lx - 1, yi = c.xy[2 * i + 1] + c.Ly - 1;
-    const double *gi = G + i, *gj = G + (size_t)i * ldg;
+  __syncthreads();
+  const int H = N >> 1, per = (H + Z2_WARPS - 1) / Z2_WARPS;
+  const int d0 = 1 + warp * per, d1 = min(H, d0 + per - 1);
+  for (int i = lane; i < N; i += 32) {
+    double s1 = 0.0, s2 = 0.0, s3 = 0.0, s4 = 0.0;
+    int j = i + d0;
+    if (j >= N) j -= N;
 #pragma unroll 4
-    for (int j = j0; j < j1; ++j) {
-      const double gij = gi[(size_t)j * ldg], gji = gj[j];
-      const double nj = 1.0 - G[j + (size_t)j * ldg];
-      const double dl = (i == j) ? 1.0 : 0.0;
-      const double pq = dl - gij;
-      v[1] += pq * pq;
-      const double a = ni * nj;
-      const double ex = (dl - gji) * gij;
-      double dc = a - ex;
-      dc = (dc + a) - ex;
-      dc = (dc + a) + a;
-      const double ph = sti * c.stag[j];
-      const int dx = xi - c.xy[2 * j], dy = yi - c.xy[2 * j + 1];
-      const double ps = c.pshift[dx + dy * W];
-      v[2] += ph * dc;
-      v[3] += ps * dc;
+    for (int d = d0; d <= d1; ++d) {
+      const double w = d == H ? 0.5 : 1.0;
+      const double a = G[i + (size_t)j * ldg], b = G[j + (size_t)i * ldg];
+      const double t = w * a * b;
+      s1 = fma(w * a, a, fma(w * b, b, s1));
+      s2 = fma(st[j], t, s2);
+      s3 = fma(pc[j], t, s3);
+      s4 = fma(ps[j], t, s4);
+      if (++j == N) j = 0;
     }
+    v[2] += s1;
+    v[6] = fma(4.0 * st[i], s2, v[6]);
+    v[7] = fma(4.0 * pc[i], s3, fma(4.0 * ps[i], s4, v[7]));
   }
-  blk_sum_n<5>(v, s.red);
-  if (threadIdx.x == 0) {
+  blk_sum_n<8>(v, s.red);
+  if (tid == 0) {
     const double flux = v[0] / (double)N;
     acc_add(c, A_FLUX_SUM, flux);
     acc_add(c, A_FLUX_SQ, flux * flux);
-    acc_add(c, A_PAIR, v[1]);
-    acc_add(c, A_CDW, v[2]);
-    acc_add(c, A_CDWS, v[3]);
-    acc_add(c, A_DENS, v[4] / (double)N);
+    acc_add(c, A_PAIR, v[2]);
+    acc_add(c, A_CDW, fma(4.0 * v[3], v[3], v[6]));
+    acc_add(c, A_CDWS, fma(4.0 * v[4], v[4], fma(4.0 * v[5], v[5], v[7])));
+    acc_add(c, A_DENS, v[1] / (double)N);
     acc_add(c, A_NOBS, 1.0);
   }
   __syncthreads();
+}
+__device__ __forceinline__ void obs_equal(const ChainDesc &c, const Smem &s, int nt) {
+  if (c.g_in_smem) obs_equal_on<true>(c, s, nt);
+  else obs_equal_on<false>(c, s, nt);
 }
 
 // ---------------------------------------------------------------------------

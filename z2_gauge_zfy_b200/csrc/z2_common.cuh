@@ -59,8 +59,8 @@ struct ChainDesc {
   int flush_shape;  // tile shape of the rank-2k flush (FS_*; 0 = by divisibility)
   int stab_exact;   // 1: the reference's column-pivoted QR in the wraps; 0: the
                     // pre-pivoted blocked QR and scale-split G (z2_stab.cuh)
-  int kin_fused;    // L when the bond table has the square-lattice layout of
-                    // kin_rows_fused / kin_cols_fused (host-checked), else 0
+  int kin_lines;    // the bond table has the layout of the line sweeps and both
+                    // line lengths are instantiated (host-checked)
   // lattice tables (device)
   const int *bonds;     // [2N][2] endpoints (0-based sites)
   const int *groups;    // [4][half] bond ids of checkerboard groups 1..4
@@ -71,7 +71,7 @@ struct ChainDesc {
   const double *chsh;   // [2N][2] cosh(alpha_b), sinh(alpha_b)
   const double *dlt;    // [2N][2] Delta(1,1), Delta(1,2) for sigma_new = +1
   const double *stag;   // [N] staggered sign
-  const double *pshift; // [(2Lx-1)(2Ly-1)] cos(qx dx + pi dy)
+  const double *phase;  // [N][2] (-1)^y cos(qx x), (-1)^y sin(qx x)
   // state (device)
   signed char *sigma;   // [Ltrot][2N]
   double *G, *UR, *VR, *DR, *ULT, *VL, *DL;      // ULT = UL^T
@@ -109,10 +109,10 @@ struct Smem {
   double *vec;      // [8N]: tau, vn1, vn2, D, dtmp, ...
   int *ivec;        // [2N]: jpvt, ...
   int *tp;          // [2N][2] slice rotation table (p1, p2) in group order
-  double *tc;       // [2N] C of the slice table
-  double *ts;       // [2N] S of the slice table (for nflag = +1)
+  double2 *cs;      // [2N] C, S of the slice table (S for nflag = +1)
+  short *gid;       // [2N] bond of a table slot, bit 14: sinh < 0
   int *bond;        // [2N][2] bond endpoints
-  signed char *sig; // [2N] sigma of the current slice
+  signed char *sig; // [2N] sigma of the slice of proposals
   int *flag;        // [16] scalars
   double *arena;    // big region
   double *G;        // G (smem arena or global)
@@ -204,9 +204,5 @@ __device__ __forceinline__ long long ph_now() { return clock64(); }
 // fragment load).
 __host__ __device__ __forceinline__ int z2_ldx(int N) { return ((N + 15) & ~15) + 4; }
 
-// ranf multiplier powers IP^i mod 2^31, i = 0..32 (filled by the host).
-__constant__ unsigned int c_ipow[33];
-
-__device__ __forceinline__ unsigned int ranf_adv(unsigned int s, int n) {
-  return (unsigned int)(((unsigned long long)s * c_ipow[n]) & 0x7fffffffull);
-}
+// One ranf draw: IP = 48828125, modulus 2^31 (which divides 2^32).
+__device__ __forceinline__ unsigned int ranf_next(unsigned int s) { return (s * 48828125u) & 0x7fffffffu; }

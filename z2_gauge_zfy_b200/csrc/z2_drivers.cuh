@@ -172,9 +172,7 @@ __device__ __noinline__ void sweep_L(const ChainDesc &c, const Smem &s) {
     { PhTimer t(c, PH_PROP); propose_slice(c, s, nt, true, 0); }   // bonds 2N..1
     {
       PhTimer t(c, PH_KIN);
-      build_table(c, s, nt);
-      kin_cols(c, s, s.G, s.ldg, N, 1);             // G B
-      kin_rows(c, s, s.G, s.ldg, N, -1);            // B^-1 G
+      kin_slices(c, s, s.G, s.ldg, nt, nt, 1, -1, 1);   // B^-1 G B
     }
     if (pd.lo > pd.hi) { pd.lo = nt; pd.hi = nt; } else pd.lo = nt;
   }
@@ -196,9 +194,7 @@ __device__ __noinline__ void sweep_R(const ChainDesc &c, const Smem &s, bool tog
     if (nt % c.Nwrap == 0) prefetch_wrap(c, nt / c.Nwrap, false);
     {
       PhTimer t(c, PH_KIN);
-      build_table(c, s, nt);
-      kin_rows(c, s, s.G, s.ldg, N, 1);             // B G
-      kin_cols(c, s, s.G, s.ldg, N, -1);            // G B^-1
+      kin_slices(c, s, s.G, s.ldg, nt, nt, 1, 1, -1);   // B G B^-1
     }
     { PhTimer t(c, PH_PROP); propose_slice(c, s, nt, false, 1); }  // bonds 1..2N
     if (pd.lo > pd.hi) { pd.lo = nt; pd.hi = nt; } else pd.hi = nt;
@@ -235,8 +231,6 @@ __device__ __noinline__ void sweep_reset(const ChainDesc &c, bool toggle, bool h
 __device__ __noinline__ void chain_sweep(const ChainDesc &c, const Smem &s, int nsweep, bool toggle,
                             double h_is_zero) {
   sweep_reset(c, toggle, h_is_zero != 0.0);
-  for (int i = threadIdx.x; i < 2 * c.nb; i += Z2_NT) s.bond[i] = c.bonds[i];
-  __syncthreads();
   load_G(c, s);
   for (int n = 0; n < nsweep; ++n) {
     if (c.acc[A_NOTBETA] == 0.0) {   // is_beta: L then R
@@ -327,7 +321,7 @@ __device__ __noinline__ void chain_therm(const ChainDesc &c, const Smem &s, int 
           const int is = (int)(-2.0 * tmp_old + 4.0) >> 2;
           const double tn = s_old * ((double)sp[b] + (double)sn[b]);
           const int it = (int)(-2.0 * tn + 4.0) >> 2;
-          st = ranf_adv(st, 1);
+          st = ranf_next(st);
           if (c.rb[is * 3 + it] > (double)st * (1.0 / 2147483648.0)) {
             sg[b] = (signed char)(-sg[b]);
             ++num;
@@ -351,7 +345,7 @@ __device__ __noinline__ void chain_therm(const ChainDesc &c, const Smem &s, int 
 // ---------------------------------------------------------------------------
 // nranf (src/calc_basic.f90:113-121): nint(ranf*N + 0.5) clamped to 1..N.
 __device__ __forceinline__ int dev_nranf(unsigned int &st, int N) {
-  st = ranf_adv(st, 1);
+  st = ranf_next(st);
   const double x = (double)st * (1.0 / 2147483648.0) * (double)N + 0.5;
   long long n = llround(x);            // nint: half away from zero
   if (n < 1) n = 1;
@@ -435,9 +429,7 @@ __device__ __noinline__ void sweep_L_trial(const ChainDesc &c, const Smem &s, in
     global_flip_slice(c, s, nt, b, lrf);
     {
       PhTimer t(c, PH_KIN);
-      build_table(c, s, nt);
-      kin_cols(c, s, s.G, s.ldg, N, 1);
-      kin_rows(c, s, s.G, s.ldg, N, -1);
+      kin_slices(c, s, s.G, s.ldg, nt, nt, 1, -1, 1);
     }
     if (pd.lo > pd.hi) { pd.lo = nt; pd.hi = nt; } else pd.lo = nt;
   }
@@ -453,9 +445,7 @@ __device__ __noinline__ void sweep_R_trial(const ChainDesc &c, const Smem &s, in
   for (int nt = 1; nt <= c.Ltrot; ++nt) {
     {
       PhTimer t(c, PH_KIN);
-      build_table(c, s, nt);
-      kin_rows(c, s, s.G, s.ldg, N, 1);
-      kin_cols(c, s, s.G, s.ldg, N, -1);
+      kin_slices(c, s, s.G, s.ldg, nt, nt, 1, 1, -1);
     }
     global_flip_slice(c, s, nt, b, lrf);
     if (pd.lo > pd.hi) { pd.lo = nt; pd.hi = nt; } else pd.hi = nt;
@@ -467,8 +457,6 @@ __device__ __noinline__ void sweep_R_trial(const ChainDesc &c, const Smem &s, in
 // Global_sweep (src/global_update.f90:320-337): nglobal Wolff moves.
 __device__ __noinline__ void chain_global(const ChainDesc &c, const Smem &s, int nglobal) {
   const int L = c.Ltrot, nb = c.nb;
-  for (int i = threadIdx.x; i < 2 * nb; i += Z2_NT) s.bond[i] = c.bonds[i];
-  __syncthreads();
   double *gs = s.red + 40;   // [0] bond, [1] size, [2] log ratio space, [3] accept
   int num = 0;
   double size_sum = 0.0;
@@ -490,7 +478,7 @@ __device__ __noinline__ void chain_global(const ChainDesc &c, const Smem &s, int
           if (c.gmask[nbr]) continue;
           if (c.sigma[(size_t)nbr * nb + b] == c.sigma[(size_t)cur * nb + b]) {
             if (c.ptime > 0.0) {
-              st = ranf_adv(st, 1);
+              st = ranf_next(st);
               if ((double)st * (1.0 / 2147483648.0) < c.ptime) {
                 c.gqueue[tail++] = nbr;
                 c.gmask[nbr] = 1;
@@ -526,7 +514,7 @@ __device__ __noinline__ void chain_global(const ChainDesc &c, const Smem &s, int
     else sweep_R_trial(c, s, b, lrf);
     if (threadIdx.x == 0) {
       const double lrt = lrf + gs[2];
-      unsigned int st = ranf_adv(*c.rng, 1);
+      unsigned int st = ranf_next(*c.rng);
       *c.rng = st;
       const double r = (double)st * (1.0 / 2147483648.0);
       const bool acc = fmin(0.0, lrt) >= log(fmax(r, 1.0e-300));
@@ -564,25 +552,114 @@ __device__ __noinline__ void chain_global(const ChainDesc &c, const Smem &s, int
 // d/dt_b = sum over the two occurrences of b in each slice of
 //   (dtau/2) sigma_b Tr[(I - G_F) X_b] = -(dtau/2) sigma_b (G_F(p1,p2) + G_F(p2,p1)),
 // G_F the Green's function whose product starts at factor F; walking the
-// factors one at a time is G <- F G F^-1.  UDV checkpoints every Nwrap slices
+// factors is G <- F G F^-1.  The factors of a slice run as the three sweeps of
+// the propagator, and the G_F between them that a bond needs follow from the
+// states before and after a sweep on the bond's own sites (grad_groups).  UDV checkpoints every Nwrap slices
 // (the L stacks from a backward pass, the R chain recomputed going forward)
 // restore G at every stabilization point.  d/dmu = beta Tr(I - G(0)).
 // ---------------------------------------------------------------------------
+// One occurrence of every bond of group g from a state X of G: the bond's block
+// X(P, P), P = {p1, p2}, is read as it is (turn 0) or taken back through the
+// bond's own rotation, E^-1 X E (turn 1); a rotation of P's sites touches no
+// other entry of the block.
+__device__ __forceinline__ double grad_block(double x11, double x12, double x21, double x22, double2 k, bool back) {
+  if (back) {      // E^-1 = [[C, -S], [-S, C]] (C^2 - S^2 = 1)
+    const double a11 = fma(k.x, x11, -k.y * x21), a12 = fma(k.x, x12, -k.y * x22);
+    const double a21 = fma(k.x, x21, -k.y * x11), a22 = fma(k.x, x22, -k.y * x12);
+    x12 = fma(a11, k.y, a12 * k.x);
+    x21 = fma(a21, k.x, a22 * k.y);
+  }
+  return x12 + x21;
+}
+
+// Gradient terms whose G_F follow from state `state` of the slice (0: before
+// the first sweep, k: after sweep k): E0 | E1 E2 E3 E3 E2 E1 | E0 as
+//   state 0: first E0;  state 1: first E1 (through E1^-1), first E2, both E3
+//   (through E2, the second also through E3);  state 2: second E2 (through
+//   E2^-1), second E1;  state 3: second E0 (through E0^-1).
+// A group has one term per bond, so its bonds are spread over the threads.
+__device__ __noinline__ void grad_groups(const ChainDesc &c, const Smem &s, int nt, int state) {
+  const int ldg = s.ldg, half = c.half;
+  const double *G = s.G;
+  const double hd = -0.5 * c.dtau;
+  const signed char *sg = c.sigma + (size_t)(nt - 1) * c.nb;
+  const int2 *tp = reinterpret_cast<const int2 *>(s.tp);
+  const auto at = [&](int i, int j) { return G[i + (size_t)j * ldg]; };
+  const auto add = [&](int q, bool back) {
+    const int2 p = tp[q];
+    const double x = grad_block(at(p.x, p.x), at(p.x, p.y), at(p.y, p.x), at(p.y, p.y), s.cs[q], back);
+    const int b = c.groups[q];
+    c.grad[b] += hd * (double)sg[b] * x;
+  };
+  for (int k = threadIdx.x; k < half; k += Z2_NT) {
+    if (state == 0) {
+      add(k, false);
+    } else if (state == 1) {
+      add(half + k, true);
+      add(2 * half + k, false);
+      // group 3: the block of E2 G E2^-1 on P: each site of P with its group-2
+      // partner; slot partner[] is found from the sites' lines (y bonds: the
+      // group-2 slot of site (x, y) is (y odd ? (y - 1) / 2 : (y / 2 - 1)) Lx + x)
+      const int q3 = 3 * half + k;
+      const int2 p = tp[q3];
+      const int Lx = c.Lx, Ly = c.Ly;
+      const auto slot2 = [&](int site) {
+        const int x = site % Lx, y = site / Lx;
+        const int m = (y & 1) ? y >> 1 : ((y + Ly - 2) % Ly) >> 1;
+        return 2 * half + m * Lx + x;
+      };
+      const int qa = slot2(p.x), qb = slot2(p.y);
+      const int2 ta = tp[qa], tb = tp[qb];
+      const int pa = ta.x == p.x ? ta.y : ta.x, pb = tb.x == p.y ? tb.y : tb.x;
+      const double2 ka = s.cs[qa], kb = s.cs[qb];
+      // rows: r(site, :) = C G(site, :) + S G(partner, :), columns with -S
+      const auto el = [&](int i, int ip, double2 ki, int j, int jp, double2 kj) {
+        const double u = fma(ki.x, at(i, j), ki.y * at(ip, j));
+        const double w = fma(ki.x, at(i, jp), ki.y * at(ip, jp));
+        return fma(u, kj.x, -w * kj.y);
+      };
+      double x11, x12, x21, x22;
+      x11 = el(p.x, pa, ka, p.x, pa, ka);
+      x12 = el(p.x, pa, ka, p.y, pb, kb);
+      x21 = el(p.y, pb, kb, p.x, pa, ka);
+      x22 = el(p.y, pb, kb, p.y, pb, kb);
+      const double2 k3 = s.cs[q3];
+      const double x = (x12 + x21) + grad_block(x11, x12, x21, x22, make_double2(k3.x, -k3.y), true);
+      const int b = c.groups[q3];
+      c.grad[b] += hd * (double)sg[b] * x;
+    } else if (state == 2) {
+      add(2 * half + k, true);
+      add(half + k, false);
+    } else {
+      add(k, true);
+    }
+  }
+  __syncthreads();
+}
+
 __device__ __noinline__ void chain_logdet_grad(const ChainDesc &c, const Smem &s) {
   const int N = c.N;
-  for (int i = threadIdx.x; i < 2 * c.nb; i += Z2_NT) s.bond[i] = c.bonds[i];
   for (int b = threadIdx.x; b < c.nb; b += Z2_NT) c.grad[b] = 0.0;
   __syncthreads();
   chain_pre(c, s);
-  // log|det(1 + UR DR VR)| = log|det(UR^T + DR VR)| = sum log D of its QRP
+  // log|det(1 + UR DR VR)| = log|det(UR^T + DR VR)|
+  //   = sum log DRb + log|det(DRb^-1 UR^T + DRs VR)|, the latter by QR (by the
+  // pivoted QR above the panel kernels' range)
   {
     int lda; double *A = qr_matrix(c, s, lda);
-    for (int j = threadIdx.x / 32; j < N; j += Z2_WARPS)
-      for (int i = threadIdx.x & 31; i < N; i += 32)
-        A[i + (size_t)j * lda] = c.UR[j + (size_t)i * N] + c.DR[i] * c.VR[i + (size_t)j * N];
-    __syncthreads();
-    blk_geqp3(A, lda, N, s.ivec, s.vec, s.vec + N, s.vec + 2 * N);
+    const bool panels = wy_ok(N, s.tile_doubles);
     double l = 0.0;
+    if (panels)
+      for (int i = threadIdx.x; i < N; i += Z2_NT) l += log(fmax(c.DR[i], 1.0));
+    blk_walk<8, double2>(
+        N, N, [&](int j, int i) { return make_double2(c.UR[j + (size_t)i * N], c.VR[i + (size_t)j * N]); },
+        [&](double2 v, int j, int i) {
+          const double d = c.DR[i], b = panels ? fmax(d, 1.0) : 1.0;
+          A[i + (size_t)j * lda] = panels ? fma(fmin(d, 1.0), v.y, v.x / b) : v.x + d * v.y;
+        });
+    __syncthreads();
+    if (panels) qr_panels_any(A, lda, N, s.vec, s.tile);
+    else blk_geqp3(A, lda, N, s.ivec, s.vec, s.vec + N, s.vec + 2 * N);
     for (int i = threadIdx.x; i < N; i += Z2_NT) l += log(fabs(A[i + (size_t)i * lda]));
     l = blk_sum(l, s.red);
     if (threadIdx.x == 0) c.acc[A_LOGDET] = l;
@@ -594,9 +671,7 @@ __device__ __noinline__ void chain_logdet_grad(const ChainDesc &c, const Smem &s
   for (int nt = c.Ltrot; nt >= 1; --nt) {
     if (nt % c.Nwrap == 0) wrap_L(c, s, nt, pd, false);
     scale_G_mu(c, s);
-    build_table(c, s, nt);
-    kin_cols(c, s, s.G, s.ldg, N, 1);
-    kin_rows(c, s, s.G, s.ldg, N, -1);
+    kin_slices(c, s, s.G, s.ldg, nt, nt, 1, -1, 1);
     if (pd.lo > pd.hi) { pd.lo = nt; pd.hi = nt; } else pd.lo = nt;
   }
   wrap_L(c, s, 0, pd, false);
@@ -610,21 +685,13 @@ __device__ __noinline__ void chain_logdet_grad(const ChainDesc &c, const Smem &s
   // forward pass with factor-by-factor wraps
   pd.lo = 1; pd.hi = 0;
   wrap_R(c, s, 0, pd, false);
-  const double hd = 0.5 * c.dtau;
   for (int nt = 1; nt <= c.Ltrot; ++nt) {
     build_table(c, s, nt);
-    for (int p = 0; p < 8; ++p) {
-      const int g = c_gorder[p];
-      for (int k = threadIdx.x; k < c.half; k += Z2_NT) {
-        const int q = g * c.half + k;
-        const int b = c.groups[q];
-        const int p1 = s.tp[2 * q], p2 = s.tp[2 * q + 1];
-        const double sgm = (double)c.sigma[(size_t)(nt - 1) * c.nb + b];
-        c.grad[b] += hd * sgm * (-(s.G[p1 + (size_t)p2 * s.ldg] + s.G[p2 + (size_t)p1 * s.ldg]));
-      }
-      __syncthreads();
-      kin_group_rows(c, s, s.G, s.ldg, N, g, 1);
-      kin_group_cols(c, s, s.G, s.ldg, N, g, -1);
+    grad_groups(c, s, nt, 0);
+    for (int k = 0; k < 3; ++k) {
+      kin_apply<true>(c, s, s.G, s.ldg, N, 1, k, k + 1);
+      kin_apply<false>(c, s, s.G, s.ldg, N, -1, k, k + 1);
+      grad_groups(c, s, nt, k + 1);
     }
     if (pd.lo > pd.hi) { pd.lo = nt; pd.hi = nt; } else pd.hi = nt;
     scale_G_mu(c, s);
