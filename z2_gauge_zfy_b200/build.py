@@ -2,7 +2,8 @@
 
     python -m z2_gauge_zfy_b200.build
 
-compiles ``csrc/z2_api.cu`` into ``libz2dqmc.so`` next to this file.
+compiles ``csrc/z2_api.cu`` and ``csrc/z2_small.cu`` into ``libz2dqmc.so`` next to
+this file.
 """
 from __future__ import annotations
 
@@ -12,10 +13,15 @@ import subprocess
 import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-SRC = os.path.join(HERE, "csrc", "z2_api.cu")
+# translation units and their own flags (the 128-thread build of the chain
+# kernel shares an SM between four blocks: 128 registers a thread)
+UNITS = (("z2_api.cu", []), ("z2_small.cu", ["-maxrregcount=128"]))
 OUT = os.path.join(HERE, "libz2dqmc.so")
-NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo",
-              "-std=c++17", "-rdc=true", "-shared", "-Xcompiler", "-fPIC"]
+# Relocatable device code: ptxas optimises a whole program's call graph at
+# once, and for this one that took over ten minutes; function by function it
+# takes half a minute.
+ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
+NVCC_FLAGS = [*ARCH, "-O3", "-lineinfo", "-std=c++17", "-dc", "-Xcompiler", "-fPIC"]
 
 
 def nvcc() -> str:
@@ -63,11 +69,24 @@ def build(force: bool = False, verbose: bool = False) -> str:
         # per-process temporary name: ranks that start together on a fresh
         # checkout may build side by side; os.replace makes the swap atomic
         tmp = f"{OUT}.tmp.{os.getpid()}"
-        cmd = [nvcc(), *NVCC_FLAGS, "-o", tmp, SRC]
-        if verbose:
-            cmd.insert(1, "-Xptxas=-v")
-            print(" ".join(cmd), flush=True)
-        subprocess.run(cmd, check=True)
+        objs, procs = [], []
+        for name, flags in UNITS:
+            objs.append(f"{tmp}.{name}.o")
+            cmd = [nvcc(), *NVCC_FLAGS, *flags, "-o", objs[-1], os.path.join(HERE, "csrc", name)]
+            if verbose:
+                cmd.insert(1, "-Xptxas=-v")
+                print(" ".join(cmd), flush=True)
+            procs.append((cmd, subprocess.Popen(cmd)))
+        try:
+            for cmd, p in procs:
+                if p.wait() != 0:
+                    raise subprocess.CalledProcessError(p.returncode, cmd)
+            subprocess.run([nvcc(), *ARCH, "-shared", "-o", tmp, *objs], check=True)
+        finally:
+            for (cmd, p), o in zip(procs, objs):
+                p.wait()
+                if os.path.exists(o):
+                    os.remove(o)
         os.replace(tmp, OUT)
     build_driver(force)
     return OUT

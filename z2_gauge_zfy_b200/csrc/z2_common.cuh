@@ -8,8 +8,13 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+// Threads of a chain's block: 256, or 128 in the build for launches of many small
+// lattices (z2_small.cu), which holds lattices up to Z2_NMAX sites only.
+#ifndef Z2_NT
 #define Z2_NT 256
+#endif
 #define Z2_WARPS (Z2_NT / 32)
+#define Z2_NMAX (Z2_NT == 256 ? 1024 : 64)
 #define Z2_FULL 0xffffffffu
 #define Z2_NRED 64              // doubles of block-reduction scratch
 

@@ -134,10 +134,12 @@ template <bool VA, bool VB, int TRI>
 __device__ __forceinline__ void gemm_sized(int n, MatRef A, const int *rowmap, MatRef B, const GemmOut &out) {
   const int t = (n + 7) >> 3;
   if (t <= 5) gemm_units<1, 2, VA, VB, TRI>(n, A, rowmap, B, out);
-  else if (t <= 8) gemm_units<2, 2, VA, VB, TRI>(n, A, rowmap, B, out);
-  else if (t <= 12) gemm_units<3, 3, VA, VB, TRI>(n, A, rowmap, B, out);
-  else if (t <= 14) gemm_units<2, 7, VA, VB, TRI>(n, A, rowmap, B, out);
-  else gemm_units<3, 9, VA, VB, TRI>(n, A, rowmap, B, out);
+  else if (Z2_NMAX <= 64 || t <= 8) gemm_units<2, 2, VA, VB, TRI>(n, A, rowmap, B, out);
+  else if constexpr (Z2_NMAX > 64) {
+    if (t <= 12) gemm_units<3, 3, VA, VB, TRI>(n, A, rowmap, B, out);
+    else if (t <= 14) gemm_units<2, 7, VA, VB, TRI>(n, A, rowmap, B, out);
+    else gemm_units<3, 9, VA, VB, TRI>(n, A, rowmap, B, out);
+  }
 }
 
 // The product in units that cut the (N / 8)^2 tiles into a multiple of the four

@@ -305,8 +305,12 @@ __device__ __forceinline__ void kin_slices(const ChainDesc &c, const Smem &s, do
       case 4: kin_square<4>(c, s, M, ld, t0, t1, dt, rf, cf); return;
       case 6: kin_square<6>(c, s, M, ld, t0, t1, dt, rf, cf); return;
       case 8: kin_square<8>(c, s, M, ld, t0, t1, dt, rf, cf); return;
-      case 10: kin_square<10>(c, s, M, ld, t0, t1, dt, rf, cf); return;
-      case 12: kin_square<12>(c, s, M, ld, t0, t1, dt, rf, cf); return;
+      case 10:
+        if constexpr (Z2_NMAX > 64) { kin_square<10>(c, s, M, ld, t0, t1, dt, rf, cf); return; }
+        break;
+      case 12:
+        if constexpr (Z2_NMAX > 64) { kin_square<12>(c, s, M, ld, t0, t1, dt, rf, cf); return; }
+        break;
       default: break;
     }
   }

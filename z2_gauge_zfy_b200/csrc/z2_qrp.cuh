@@ -397,6 +397,7 @@ __device__ __noinline__ void qrp_reg(double *A, int lda, int n, int *jpvt, doubl
 __device__ __forceinline__ void blk_geqp3_fast(double *A, int lda, int n, int *jpvt, double *tau,
                                                double *vn1, double *vn2, double *work, int wd,
                                                double *red) {
+#if Z2_NT == 256   // the register tile is 16 x 16 threads
   if (work != nullptr && wd >= 2 * n) {
     switch ((n + 15) >> 4) {
       case 1: qrp_reg<1>(A, lda, n, jpvt, tau, vn1, vn2, work, red); return;
@@ -411,5 +412,6 @@ __device__ __forceinline__ void blk_geqp3_fast(double *A, int lda, int n, int *j
       default: break;
     }
   }
+#endif
   blk_geqp3_tc(A, lda, n, jpvt, tau, vn1, vn2);
 }

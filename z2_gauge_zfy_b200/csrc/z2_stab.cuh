@@ -149,7 +149,8 @@ __device__ __forceinline__ bool wy_ok(int n, int wd) {
 }
 
 __device__ __forceinline__ void qr_panels_any(double *A, int lda, int n, double *vd, double *work) {
-  if (__isShared(A) && n <= 160) blk_qr_panels<true, 5>(A, lda, n, vd, work);
+  if constexpr (Z2_NMAX <= 64) blk_qr_panels<true, 2>(A, lda, n, vd, work);
+  else if (__isShared(A) && n <= 160) blk_qr_panels<true, 5>(A, lda, n, vd, work);
   else blk_qr_panels<false, 8>(A, lda, n, vd, work);
 }
 __device__ __forceinline__ void form_q_any(double *A, int lda, int n, const double *vd, double *work) {
@@ -157,7 +158,10 @@ __device__ __forceinline__ void form_q_any(double *A, int lda, int n, const doub
   else blk_form_q<false>(A, lda, n, vd, work);
 }
 __device__ __forceinline__ void gj_any(double *M, int ldm, int n, int *piv, double *work) {
-  if (__isShared(M) && n <= 160) {
+  if constexpr (Z2_NMAX <= 64) {
+    if (n <= 32) blk_gj_panels<true, 1>(M, ldm, n, piv, work);
+    else blk_gj_panels<true, 2>(M, ldm, n, piv, work);
+  } else if (__isShared(M) && n <= 160) {
     if (n <= 32) blk_gj_panels<true, 1>(M, ldm, n, piv, work);
     else if (n <= 64) blk_gj_panels<true, 2>(M, ldm, n, piv, work);
     else if (n <= 96) blk_gj_panels<true, 3>(M, ldm, n, piv, work);
@@ -169,10 +173,11 @@ __device__ __forceinline__ void gj_any(double *M, int ldm, int n, int *piv, doub
 }
 
 // A <- A P S, column j of it being sc[j] (null: 1) times column perm[j] of A, in
-// shared memory through registers (n <= 32 T, n <= 8 C).
-template <int T, int C>
+// shared memory through registers (n <= 32 T).
+template <int T>
 __device__ __noinline__ void permute_cols_reg(double *A, int lda, int n, const int *perm, const double *sc) {
   A = as_shared(A);
+  constexpr int C = 32 * T / Z2_WARPS;    // columns per warp
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double v[C][T];
 #pragma unroll
@@ -196,12 +201,16 @@ __device__ __noinline__ void permute_cols_reg(double *A, int lda, int n, const i
 // The same for any A; W: an n x n global workspace.
 __device__ __forceinline__ void permute_cols(double *A, int lda, int n, const int *perm, const double *sc,
                                              double *W) {
-  if (__isShared(A) && n <= 160) {
-    if (n <= 32) permute_cols_reg<1, 4>(A, lda, n, perm, sc);
-    else if (n <= 64) permute_cols_reg<2, 8>(A, lda, n, perm, sc);
-    else if (n <= 96) permute_cols_reg<3, 12>(A, lda, n, perm, sc);
-    else if (n <= 128) permute_cols_reg<4, 16>(A, lda, n, perm, sc);
-    else permute_cols_reg<5, 20>(A, lda, n, perm, sc);
+  if constexpr (Z2_NMAX <= 64) {
+    if (n <= 32) permute_cols_reg<1>(A, lda, n, perm, sc);
+    else permute_cols_reg<2>(A, lda, n, perm, sc);
+    return;
+  } else if (__isShared(A) && n <= 160) {
+    if (n <= 32) permute_cols_reg<1>(A, lda, n, perm, sc);
+    else if (n <= 64) permute_cols_reg<2>(A, lda, n, perm, sc);
+    else if (n <= 96) permute_cols_reg<3>(A, lda, n, perm, sc);
+    else if (n <= 128) permute_cols_reg<4>(A, lda, n, perm, sc);
+    else permute_cols_reg<5>(A, lda, n, perm, sc);
     return;
   }
   blk_copy(W, n, A, lda, n, n);
