@@ -22,10 +22,13 @@ __host__ __device__ __forceinline__ int wy_ldv(int n) {
   return ((((n + 7) & ~7) + 11) & ~15) + 4;
 }
 __host__ __device__ __forceinline__ int wy_panels(int n) { return (n + WY_NB - 1) / WY_NB; }
-// Shared work space (doubles): two panel buffers and every panel's T.
+// Shared work space (doubles): two panel buffers, every panel's T, and 64 more.
 __host__ __device__ __forceinline__ int wy_work(int n) {
-  return 2 * WY_NB * wy_ldv(n) + WY_NB * WY_NB * wy_panels(n);
+  return 2 * WY_NB * wy_ldv(n) + WY_NB * WY_NB * (wy_panels(n) + 1);
 }
+
+template <int I>
+struct WyIdx { static constexpr int v = I; };
 
 // 1 / x to rounding for a normal x of moderate size: the hardware's
 // approximation and two Newton steps r <- r (2 - x r) (no special cases, so it
@@ -147,10 +150,10 @@ __device__ __forceinline__ void panel_update(double *A, int lda, int n, int j0, 
 // the reflectors below it go back into A, v(j) into vd, the reflectors clean
 // (zeros above) into Vb (column c at c ldv), and the block's T (DLARFT forward /
 // columnwise with g for tau, column-major 8 x 8) into Tb; the products
-// v_q^T v_k it needs come with the same sums.
+// v_q^T v_k it needs come with the same sums, through the 64 doubles zs.
 template <int R>
 __device__ __forceinline__ void warp_qr_panel(double *A, int lda, int n, int j0, double *Vb, int ldv,
-                                              double *Tb, double *vd) {
+                                              double *Tb, double *vd, double *zs) {
   const int lane = threadIdx.x & 31, lr = lane >> 2, lc = lane & 3;
   const int mp = n - j0, ib = mp < WY_NB ? mp : WY_NB;
   double *Ap = A + j0 + (j0 + 2 * lc) * lda + lr;
@@ -160,61 +163,62 @@ __device__ __forceinline__ void warp_qr_panel(double *A, int lda, int n, int j0,
 #pragma unroll
     for (int e = 0; e < 2; ++e)
       a[i][e] = (lr + 8 * i < mp && 2 * lc + e < ib) ? Ap[8 * i + e * lda] : 0.0;
-  double z[8][2];    // v_q^T v_k for this lane's q = 2 lc, 2 lc + 1
-  double gk[8], vk[8];
+  double gl = 0.0, vl = 1.0;    // lane k < 8: g and v(j) of column k
+  // one column; e = k % 2 is static, so that the panel is a loop over column
+  // pairs (unrolled over all eight, the panels alone filled the instruction
+  // cache)
+  const auto column = [&](int k, auto E) {
+    constexpr int e = decltype(E)::v;
+    const int own = k >> 1;
+    double x[R];
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    gk[k] = 0.0;
-    vk[k] = 1.0;
-    z[k][0] = z[k][1] = 0.0;
-    if (k < ib) {                                   // uniform
-      // column k in every lane group, rows below the diagonal, and row j
-      const int own = k >> 1, e = k & 1;
-      double x[R];
+    for (int i = 0; i < R; ++i) x[i] = __shfl_sync(Z2_FULL, a[i][e], own, 4);
+    const double alpha = __shfl_sync(Z2_FULL, x[0], 4 * k);
+    const double r0 = __shfl_sync(Z2_FULL, a[0][0], 4 * k + lc);
+    const double r1 = __shfl_sync(Z2_FULL, a[0][1], 4 * k + lc);
+    x[0] = lr > k ? x[0] : 0.0;                     // rows below the diagonal
+    double d0 = x[0] * a[0][0], d1 = x[0] * a[0][1], f0 = 0.0, f1 = 0.0;
 #pragma unroll
-      for (int i = 0; i < R; ++i) x[i] = __shfl_sync(Z2_FULL, a[i][e], own, 4);
-      const double alpha = __shfl_sync(Z2_FULL, x[0], 4 * k);
-      const double r0 = __shfl_sync(Z2_FULL, a[0][0], 4 * k + lc);
-      const double r1 = __shfl_sync(Z2_FULL, a[0][1], 4 * k + lc);
-      x[0] = lr > k ? x[0] : 0.0;
-      double d0 = x[0] * a[0][0], d1 = x[0] * a[0][1], f0 = 0.0, f1 = 0.0;
-#pragma unroll
-      for (int i = 1; i < R; ++i) {
-        if (i & 1) { f0 = fma(x[i], a[i][0], f0); f1 = fma(x[i], a[i][1], f1); }
-        else { d0 = fma(x[i], a[i][0], d0); d1 = fma(x[i], a[i][1], d1); }
-      }
-      d0 += f0; d1 += f1;
-#pragma unroll
-      for (int o = 4; o <= 16; o <<= 1) {
-        d0 += __shfl_xor_sync(Z2_FULL, d0, o);
-        d1 += __shfl_xor_sync(Z2_FULL, d1, o);
-      }
-      const double ss = __shfl_sync(Z2_FULL, e ? d1 : d0, own, 4);
-      // beta = -sign(alpha) sqrt(alpha^2 + |x|^2); a zero column: H = I
-      const bool refl = ss != 0.0;
-      const double q = refl ? fma(alpha, alpha, ss) : 1.0;
-      double nb, gq;
-      sqrt_rcp(q, fabs(alpha), nb, gq);
-      const double beta = refl ? -copysign(nb, alpha) : alpha;
-      const double hv = alpha - beta;
-      const double g = refl ? gq : 0.0;
-      // v_c^T v_k for the earlier columns, H_j on the later ones:
-      // A(:, c) -= g (v(j) A(j, c) + x^T A(j+1:, c)) v
-      const double p0 = fma(hv, r0, d0), p1 = fma(hv, r1, d1);
-      z[k][0] = p0;
-      z[k][1] = p1;
-      const double w0 = 2 * lc > k ? -g * p0 : 0.0, w1 = 2 * lc + 1 > k ? -g * p1 : 0.0;
-      x[0] = lr == k ? hv : x[0];
-#pragma unroll
-      for (int i = 0; i < R; ++i) {
-        a[i][0] = fma(w0, x[i], a[i][0]);
-        a[i][1] = fma(w1, x[i], a[i][1]);
-      }
-      if (lr == k && lc == own) a[0][e] = beta;
-      gk[k] = g;
-      vk[k] = hv;
+    for (int i = 1; i < R; ++i) {
+      if (i & 1) { f0 = fma(x[i], a[i][0], f0); f1 = fma(x[i], a[i][1], f1); }
+      else { d0 = fma(x[i], a[i][0], d0); d1 = fma(x[i], a[i][1], d1); }
     }
+    d0 += f0; d1 += f1;
+#pragma unroll
+    for (int o = 4; o <= 16; o <<= 1) {
+      d0 += __shfl_xor_sync(Z2_FULL, d0, o);
+      d1 += __shfl_xor_sync(Z2_FULL, d1, o);
+    }
+    const double ss = __shfl_sync(Z2_FULL, e ? d1 : d0, own, 4);
+    // beta = -sign(alpha) sqrt(alpha^2 + |x|^2); a zero column: H = I
+    const bool refl = ss != 0.0;
+    const double q = refl ? fma(alpha, alpha, ss) : 1.0;
+    double nb, gq;
+    sqrt_rcp(q, fabs(alpha), nb, gq);
+    const double beta = refl ? -copysign(nb, alpha) : alpha;
+    const double hv = alpha - beta;
+    const double g = refl ? gq : 0.0;
+    // v_c^T v_k for the earlier columns, H_j on the later ones:
+    // A(:, c) -= g (v(j) A(j, c) + x^T A(j+1:, c)) v
+    const double p0 = fma(hv, r0, d0), p1 = fma(hv, r1, d1);
+    if (lr == 0) { zs[8 * k + 2 * lc] = p0; zs[8 * k + 2 * lc + 1] = p1; }
+    const double w0 = 2 * lc > k ? -g * p0 : 0.0, w1 = 2 * lc + 1 > k ? -g * p1 : 0.0;
+    x[0] = lr == k ? hv : x[0];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      a[i][0] = fma(w0, x[i], a[i][0]);
+      a[i][1] = fma(w1, x[i], a[i][1]);
+    }
+    if (lr == k && lc == own) a[0][e] = beta;
+    if (lane == k) { gl = g; vl = hv; }
+  };
+#pragma unroll 1
+  for (int k = 0; k < ib; k += 2) {
+    column(k, WyIdx<0>{});
+    if (k + 1 < ib) column(k + 1, WyIdx<1>{});
   }
+  for (int t = 8 * ib + lane; t < 64; t += 32) zs[t] = 0.0;   // columns past the matrix
+  __syncwarp();
   const int m8 = (mp + 7) & ~7;
 #pragma unroll
   for (int i = 0; i < R; ++i) {
@@ -230,12 +234,9 @@ __device__ __forceinline__ void warp_qr_panel(double *A, int lda, int n, int j0,
       if (r < m8 && (i > 0 || r != c)) Vb[j0 + r + c * ldv] = v;
     }
   }
-  if (lane == 0) {
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      Vb[j0 + c + c * ldv] = c < ib ? vk[c] : 0.0;
-      if (c < ib) vd[j0 + c] = vk[c];
-    }
+  if (lane < 8) {
+    Vb[j0 + lane + lane * ldv] = lane < ib ? vl : 0.0;
+    if (lane < ib) vd[j0 + lane] = vl;
   }
   // T row by row in lane i < 8: T(i, k) = -g_k sum_{q < k} T(i, q) z_q(k)
   double tr[8];
@@ -243,8 +244,9 @@ __device__ __forceinline__ void warp_qr_panel(double *A, int lda, int n, int j0,
   for (int k = 0; k < 8; ++k) {
     double s = 0.0;
 #pragma unroll
-    for (int q = 0; q < k; ++q) s = fma(tr[q], __shfl_sync(Z2_FULL, z[k][q & 1], q >> 1), s);
-    tr[k] = lane == k ? gk[k] : (lane < k ? -gk[k] * s : 0.0);
+    for (int q = 0; q < k; ++q) s = fma(tr[q], zs[8 * k + q], s);
+    const double g = __shfl_sync(Z2_FULL, gl, k);
+    tr[k] = lane == k ? g : (lane < k ? -g * s : 0.0);
   }
   if (lane < 8) {
 #pragma unroll
@@ -256,19 +258,20 @@ __device__ __forceinline__ void warp_qr_panel(double *A, int lda, int n, int j0,
 // The panel with the smallest R that holds its n - j0 <= 32 T rows.
 template <bool SH, int T>
 __device__ __noinline__ void warp_qr_panel_any(double *A, int lda, int n, int j0, double *Vb, int ldv,
-                                               double *Tb, double *vd) {
+                                               double *Tb, double *vd, double *zs) {
   if (SH) A = as_shared(A);
+  zs = as_shared(zs);
   Vb = as_shared(Vb);
   Tb = as_shared(Tb);
   vd = as_shared(vd);
   const int mp = n - j0;
-  if (T > 5 && mp > 160) warp_qr_panel<32>(A, lda, n, j0, Vb, ldv, Tb, vd);
-  else if (T > 4 && mp > 144) warp_qr_panel<20>(A, lda, n, j0, Vb, ldv, Tb, vd);
-  else if (T > 3 && mp > 104) warp_qr_panel<18>(A, lda, n, j0, Vb, ldv, Tb, vd);
-  else if (T > 2 && mp > 64) warp_qr_panel<13>(A, lda, n, j0, Vb, ldv, Tb, vd);
-  else if (T > 1 && mp > 32) warp_qr_panel<8>(A, lda, n, j0, Vb, ldv, Tb, vd);
-  else if (mp > 16) warp_qr_panel<4>(A, lda, n, j0, Vb, ldv, Tb, vd);
-  else warp_qr_panel<2>(A, lda, n, j0, Vb, ldv, Tb, vd);
+  if (T > 5 && mp > 160) warp_qr_panel<32>(A, lda, n, j0, Vb, ldv, Tb, vd, zs);
+  else if (T > 4 && mp > 144) warp_qr_panel<20>(A, lda, n, j0, Vb, ldv, Tb, vd, zs);
+  else if (T > 3 && mp > 104) warp_qr_panel<18>(A, lda, n, j0, Vb, ldv, Tb, vd, zs);
+  else if (T > 2 && mp > 64) warp_qr_panel<13>(A, lda, n, j0, Vb, ldv, Tb, vd, zs);
+  else if (T > 1 && mp > 32) warp_qr_panel<8>(A, lda, n, j0, Vb, ldv, Tb, vd, zs);
+  else if (mp > 16) warp_qr_panel<4>(A, lda, n, j0, Vb, ldv, Tb, vd, zs);
+  else warp_qr_panel<2>(A, lda, n, j0, Vb, ldv, Tb, vd, zs);
 }
 
 // C <- C - V (op(T) (V^T C)) for NT tiles of 8 columns of A, rows j0..n, by one
@@ -352,8 +355,8 @@ __device__ __noinline__ void blk_qr_panels(double *A, int lda, int n, double *vd
   work = as_shared(work);
   const int warp = threadIdx.x >> 5;
   const int ldv = wy_ldv(n), np = wy_panels(n);
-  double *Tall = work + 2 * WY_NB * ldv;
-  if (warp == 0) warp_qr_panel_any<SH, T>(A, lda, n, 0, work, ldv, Tall, vd);
+  double *Tall = work + 2 * WY_NB * ldv, *zs = Tall + 64 * np;
+  if (warp == 0) warp_qr_panel_any<SH, T>(A, lda, n, 0, work, ldv, Tall, vd, zs);
   __syncthreads();
   for (int p = 0; p + 1 < np; ++p) {
     const int j0 = p * WY_NB;
@@ -362,7 +365,7 @@ __device__ __noinline__ void blk_qr_panels(double *A, int lda, int n, double *vd
     wy_tiles<true>(A, lda, n, j0, p + 1 + warp, warp == 0 ? np : Z2_WARPS - 1, np, Vb, ldv, Tb);
     if (warp == 0)
       warp_qr_panel_any<SH, T>(A, lda, n, j0 + WY_NB, work + ((p + 1) & 1) * WY_NB * ldv, ldv,
-                               Tall + (p + 1) * 64, vd);
+                               Tall + (p + 1) * 64, vd, zs);
     __syncthreads();
   }
 }
@@ -492,37 +495,60 @@ __device__ __forceinline__ unsigned warp_gj_panel(double *M, int ldm, int n, int
 #pragma unroll
     for (int c = 0; c < 8; ++c) a[t][c] = (r < n && c < ib) ? Mp[r + c * ldm] : 0.0;
   }
+  // one step on the register column K (the panel's column k)
+  const auto step = [&](int k, auto KC) {
+    constexpr int K = decltype(KC)::v;
+    unsigned key = 0;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    if (k < ib) {                                   // uniform
-      unsigned key = 0;
+    for (int t = 0; t < T; ++t) {
+      const unsigned h = ((unsigned)__double2hiint(fabs(a[t][K])) & 0xFFFFFF00u) |
+                         (unsigned)(255 - (lane + 32 * t));
+      if (!((used >> t) & 1u)) key = max(key, h);
+    }
+    key = __reduce_max_sync(Z2_FULL, key);
+    const int br = 255 - (int)(key & 0xFFu), ol = br & 31, ot = br >> 5;
+    double u[8];
+    pick_row<0, T>(ot, a, u);                       // uniform branches
+#pragma unroll
+    for (int c = 0; c < 8; ++c) u[c] = __shfl_sync(Z2_FULL, u[c], ol);
+    const double rd = rcp_newton(u[K]);
+    if (lane == 0) piv[j0 + k] = br;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) u[c] *= rd;
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+      const bool isp = t == ot && lane == ol;
+      const double l = isp ? 0.0 : a[t][K];
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        if (c != K) a[t][c] = fma(-l, u[c], a[t][c]);
+      a[t][K] = isp ? 1.0 : -l * rd;
+      if (isp) { scl[t] = rd; used |= 1u << t; }
+    }
+  };
+  if constexpr (T <= 2) {
+    // a loop over the columns, the current one rotated to the front (16 T moves
+    // a step, for an eighth of the code)
+#pragma unroll 1
+    for (int k = 0; k < 8; ++k) {
+      if (k < ib) step(k, WyIdx<0>{});
 #pragma unroll
       for (int t = 0; t < T; ++t) {
-        const unsigned h = ((unsigned)__double2hiint(fabs(a[t][k])) & 0xFFFFFF00u) |
-                           (unsigned)(255 - (lane + 32 * t));
-        if (!((used >> t) & 1u)) key = max(key, h);
-      }
-      key = __reduce_max_sync(Z2_FULL, key);
-      const int br = 255 - (int)(key & 0xFFu), ol = br & 31, ot = br >> 5;
-      double u[8];
-      pick_row<0, T>(ot, a, u);                     // uniform branches
+        const double f = a[t][0];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) u[c] = __shfl_sync(Z2_FULL, u[c], ol);
-      const double rd = rcp_newton(u[k]);
-      if (lane == 0) piv[j0 + k] = br;
-#pragma unroll
-      for (int c = 0; c < 8; ++c) u[c] *= rd;
-#pragma unroll
-      for (int t = 0; t < T; ++t) {
-        const bool isp = t == ot && lane == ol;
-        const double l = isp ? 0.0 : a[t][k];
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
-          if (c != k) a[t][c] = fma(-l, u[c], a[t][c]);
-        a[t][k] = isp ? 1.0 : -l * rd;
-        if (isp) { scl[t] = rd; used |= 1u << t; }
+        for (int c = 0; c < 7; ++c) a[t][c] = a[t][c + 1];
+        a[t][7] = f;
       }
     }
+  } else {
+    if (0 < ib) step(0, WyIdx<0>{});
+    if (1 < ib) step(1, WyIdx<1>{});
+    if (2 < ib) step(2, WyIdx<2>{});
+    if (3 < ib) step(3, WyIdx<3>{});
+    if (4 < ib) step(4, WyIdx<4>{});
+    if (5 < ib) step(5, WyIdx<5>{});
+    if (6 < ib) step(6, WyIdx<6>{});
+    if (7 < ib) step(7, WyIdx<7>{});
   }
   const int n8 = (n + 7) & ~7;
 #pragma unroll

@@ -23,8 +23,8 @@
 #pragma once
 #include "z2_linalg.cuh"
 
-// Checkerboard group order of one B (src/operator_kin.f90:74-85).
-__device__ __constant__ int c_gorder[8] = {0, 1, 2, 3, 3, 2, 1, 0};
+// Checkerboard group of pass p = 0..7 of one B (src/operator_kin.f90:74-85).
+__device__ __forceinline__ int kin_pass_group(int p) { return p < 4 ? p : 7 - p; }
 
 // The part of the slice table that does not change: position q = g half + k
 // holds bond groups[q]: its sites, C, sinh (in S's place) and, in gid, the bond
@@ -226,7 +226,7 @@ __device__ __forceinline__ void kin_groups(const ChainDesc &c, const Smem &s, do
                                            int p0, int p1) {
   for (int i = threadIdx.x; i < n; i += Z2_NT)
     for (int p = p0; p < p1; ++p)
-      kin_group_vec(s, ROWS ? M + (size_t)i * ld : M + i, ROWS ? 1 : (size_t)ld, c_gorder[p] * c.half, c.half, fl);
+      kin_group_vec(s, ROWS ? M + (size_t)i * ld : M + i, ROWS ? 1 : (size_t)ld, kin_pass_group(p) * c.half, c.half, fl);
   __syncthreads();
 }
 // Sweeps k0 <= K < k1 of M <- B^nflag M for n columns (ROWS) or M <- M B^nflag for
