@@ -27,9 +27,7 @@ __device__ __forceinline__ void gemm_unit(int n, MatRef A, MatRef B, int r0, int
   const int lb = TRI == 1 ? r0 : (TRI == 2 ? c0 : 0);
   const double *pa = A.p + (lb + 2 * lc) * A.cs, *pb = B.p + (lb + 2 * lc) * B.rs;
   const int sa = 8 * A.cs, sb = 8 * B.rs;
-#pragma unroll 1
-  for (int l = lb + 2 * lc; l < n8; l += 8) {
-    double2 fa[RT], fb[CT];
+  const auto load = [&](double2 (&fa)[RT], double2 (&fb)[CT]) {
 #pragma unroll
     for (int a = 0; a < RT; ++a)
       fa[a] = VA ? *reinterpret_cast<const double2 *>(pa + oa[a]) : make_double2(pa[oa[a]], pa[oa[a] + A.cs]);
@@ -38,6 +36,8 @@ __device__ __forceinline__ void gemm_unit(int n, MatRef A, MatRef B, int r0, int
       fb[b] = VB ? *reinterpret_cast<const double2 *>(pb + ob[b]) : make_double2(pb[ob[b]], pb[ob[b] + B.rs]);
     pa += sa;
     pb += sb;
+  };
+  const auto mul = [&](int l, double2 (&fa)[RT], double2 (&fb)[CT]) {
     if (TRI == 1) {
 #pragma unroll
       for (int a = 0; a < RT; ++a) {
@@ -62,6 +62,33 @@ __device__ __forceinline__ void gemm_unit(int n, MatRef A, MatRef B, int r0, int
     for (int a = 0; a < RT; ++a)
 #pragma unroll
       for (int b = 0; b < CT; ++b) dmma884(acc[a][b][0], acc[a][b][1], fa[a].y, fb[b].y);
+  };
+  if constexpr (Z2_NT == 256 && RT * CT >= 8 && RT * CT <= 14) {
+    // middle units: the operands of the next eight k values are in flight behind
+    // the products (an L2 latency is several times their issue time; N = 64
+    // 15 -> 12 K cycles).  The largest have no registers left for it, the
+    // smallest too few k steps.
+    int l = lb + 2 * lc;
+    const int last = n8 - 8 + 2 * lc;
+    double2 fa[2][RT], fb[2][CT];
+    if (l <= last) load(fa[0], fb[0]);
+#pragma unroll 1
+    while (l <= last) {
+      if (l + 8 <= last) load(fa[1], fb[1]);
+      mul(l, fa[0], fb[0]);
+      l += 8;
+      if (l > last) break;
+      if (l + 8 <= last) load(fa[0], fb[0]);
+      mul(l, fa[1], fb[1]);
+      l += 8;
+    }
+  } else {
+#pragma unroll 1
+    for (int l = lb + 2 * lc; l < n8; l += 8) {
+      double2 fa[RT], fb[CT];
+      load(fa, fb);
+      mul(l, fa, fb);
+    }
   }
   if (n8 < n) {              // four trailing k values
     const int l = n8 + lc;
@@ -134,7 +161,7 @@ template <bool VA, bool VB, int TRI>
 __device__ __forceinline__ void gemm_sized(int n, MatRef A, const int *rowmap, MatRef B, const GemmOut &out) {
   const int t = (n + 7) >> 3;
   if (t <= 5) gemm_units<1, 2, VA, VB, TRI>(n, A, rowmap, B, out);
-  else if (Z2_NMAX <= 64 || t <= 8) gemm_units<2, 2, VA, VB, TRI>(n, A, rowmap, B, out);
+  else if (Z2_NMAX <= 64 || t <= 8) gemm_units<2, Z2_NT == 256 ? 4 : 2, VA, VB, TRI>(n, A, rowmap, B, out);
   else if constexpr (Z2_NMAX > 64) {
     if (t <= 12) gemm_units<3, 3, VA, VB, TRI>(n, A, rowmap, B, out);
     else if (t <= 14) gemm_units<2, 7, VA, VB, TRI>(n, A, rowmap, B, out);
