@@ -62,7 +62,7 @@ class ChainSpec:
 
 # DRAM bytes (read + write) of one step of the 256-chain workload, from one
 # ncu capture of the chain kernel (dram__bytes_read.sum + dram__bytes_write.sum)
-TRAFFIC_BYTES_PER_STEP = 3254171904 + 5548485632
+TRAFFIC_BYTES_PER_STEP = 3145060352 + 5572685056
 
 
 def batched_chains(rank: int = 0, n: int = 256):
@@ -494,7 +494,7 @@ def main():
         "flush_shape": ",".join(f"N{n}:{FLUSH_SHAPES[x]}" for n, x in sorted(smap.items())),
         "tuning": "z2_tune: ranks 4..64 (shared memory caps them: k <= 8 at N = 144) x every "
                   "flush tile shape valid for N, median SM cycles of 3 probe chains, first "
-                  "within 3 % of the fastest in the order (default shape, smaller rank)",
+                  "within 5 % of the fastest in the order (default shape and rank, smaller ranks)",
         "autotune_s": t_tune,
         "bin_observables_mean": dict(zip(("flux_avg", "chi_flux", "pair_sc_q0", "cdw_pi",
                                           "cdw_shift", "cdw_ratio", "density"),

@@ -474,7 +474,7 @@ __device__ __forceinline__ void pick_row(int i, const double (&a)[T][8], double 
 // Eight exchange steps on the panel M(:, j0:j0+8) by one warp, n <= 32 T: step
 // k picks the largest entry of column k among the rows not yet used (to
 // within 2^-12 relative: the high word of |a|, which orders like the value,
-// with its low byte replaced by 255 - row / 4, ties to the smaller row),
+// with its low byte replaced by 255 - row, ties to the smaller row),
 // p with pivot d and l_r = a(r, k):
 //   a(p, :) /= d, a(r, c) -= l_r a(p, c), a(r, k) = -l_r / d, a(p, k) = 1 / d.
 // On exit the panel (in M and in Zb, rows up to the next multiple of 8) holds

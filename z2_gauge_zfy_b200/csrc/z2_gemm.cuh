@@ -172,7 +172,8 @@ __device__ __forceinline__ void gemm_sized(int n, MatRef A, const int *rowmap, M
 // The product in units that cut the (N / 8)^2 tiles into a multiple of the four
 // sub-partitions' tensor pipes where they can (18 x 18 tiles: 12 units of 3 x 9,
 // three per sub-partition), with as many products per fragment as registers
-// allow.  a_upper: A(i, l) reads as 0 for i > l; b_lower: B(l, j) reads as 0 for
+// allow: N = 144 takes 80 K cycles against 103 K for 16 x 16 groups (47 K at the
+// SM's DMMA rate; the fragment loads' trips to L2 are the rest).  a_upper: A(i, l) reads as 0 for i > l; b_lower: B(l, j) reads as 0 for
 // l < j.
 __device__ __noinline__ void gemm_nnn(int n, MatRef A, const int *rowmap, bool a_upper, MatRef B,
                                       bool b_lower, GemmOut out) {
