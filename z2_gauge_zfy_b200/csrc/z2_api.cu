@@ -1498,9 +1498,8 @@ static __device__ __align__(256) double z2_noalloc_scratch[5 * Z2_NOALLOC_NMAX *
 
 // Shared work space of the two QR steps, enough for every N <= 144 so that
 // this kernel runs the same QR code as z2_stab_green: the register-resident
-// pivoted QR needs 2N doubles, the blocked DORGQR (16-column blocks) its V and
-// W panels (4544 doubles at N = 144) and, for the T prologue, 8 warps x
-// (2 * 16^2 + 4 * 16) = 4608 doubles.
+// pivoted QR needs 2N doubles, the panel kernels wy_work(144) = 3584 doubles;
+// 4608 are kept.
 constexpr int kNoallocTile = Z2_WARPS * (2 * 16 * 16 + 4 * 16);
 
 __global__ void __launch_bounds__(Z2_NT, 1)
