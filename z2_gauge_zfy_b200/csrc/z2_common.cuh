@@ -118,7 +118,7 @@ struct Smem {
   short *gid;       // [2N] bond of a table slot, bit 14: sinh < 0
   int *bond;        // [2N][2] bond endpoints
   signed char *sig; // [2N] sigma of the slice of proposals
-  int *flag;        // [16] scalars
+  int *flag;        // [16] scalars; two sets of posts (z2_window.h) while proposing
   double *arena;    // big region
   double *G;        // G (smem arena or global)
   int ldg;          // leading dimension of G

@@ -4,6 +4,7 @@
 #pragma once
 #include "z2_blocked.cuh"
 #include "z2_flush.cuh"
+#include "z2_window.h"
 
 // 48828125^n mod 2^31 (the ranf multiplier power of the n-th draw): the low 32
 // bits of the products are enough, 2^31 divides 2^32.
@@ -29,7 +30,9 @@ __device__ __forceinline__ unsigned int ranf_pow(int n) {
 //   z = Prod^-1 Delta (I - G)(P, :) of the current G = G0 - X Yt^T join X and
 //   Yt; barrier;
 //   each thread updates its own bond's four entries, G -= u z.
-// After k accepts (or at the end of the slice) G0 -= X Yt^T.
+// After k accepts (or at the end of the slice) G0 -= X Yt^T.  A round without an
+// accept ends the window with no second barrier, so the windows post in two
+// sets of words in turn (z2_window.h).
 //
 // Bound: the latency of the round (the ratio, two barriers, the loop over the
 // queued columns), not the arithmetic.  Evaluating from X and Yt for 32
@@ -52,7 +55,6 @@ __device__ __noinline__ void propose_window(const ChainDesc &c, const Smem &s, i
   double2 *X2 = reinterpret_cast<double2 *>(as_shared(s.X));
   double2 *Y2 = reinterpret_cast<double2 *>(as_shared(s.Yt));
   double2 *slot = reinterpret_cast<double2 *>(as_shared(s.red));   // [8][2] K of the posted candidates
-  int *flag = as_shared(s.flag);                                   // [8] proposal << 20 | p1 << 10 | p2
   const int *bond = as_shared(s.bond);
   signed char *sg = c.sigma + (size_t)(nt - 1) * nb;
   const signed char *gprev = c.sigma + (size_t)((nt - 2 + Lt) % Lt) * nb;
@@ -92,6 +94,8 @@ __device__ __noinline__ void propose_window(const ChainDesc &c, const Smem &s, i
       g22 = fma(-xb.y, yb.y, fma(-xb.x, yb.x, g22));
     }
     int done = 0;
+    // the warps' candidates, proposal << 20 | p1 << 10 | p2
+    int *flag = as_shared(s.flag) + z2_window_post<Z2_NT>(base);
     for (;;) {
       const long long t0 = ph_now();
       // ---- evaluate ----
