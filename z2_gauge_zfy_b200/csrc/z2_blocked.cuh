@@ -30,9 +30,11 @@ __host__ __device__ __forceinline__ int wy_work(int n) {
 template <int I>
 struct WyIdx { static constexpr int v = I; };
 
-// 1 / x to rounding for a normal x of moderate size: the hardware's
-// approximation and two Newton steps r <- r (2 - x r) (no special cases, so it
-// schedules beside other work, unlike the division).
+// 1 / x to rounding (error < 1.01 2^-53) for 2^-1022 <= |x| <= 2^1022: the
+// hardware's approximation and two Newton steps r <- r (2 - x r) (no special
+// cases, so it schedules beside other work, unlike the division).  Outside, 0
+// and subnormals give NaN and larger values 0: the determinant of an accepted
+// proposal and the pivots of a matrix of order one do not get there.
 __device__ __forceinline__ double rcp_newton(double x) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
@@ -40,7 +42,9 @@ __device__ __forceinline__ double rcp_newton(double x) {
   return fma(r, fma(-x, r, 1.0), r);
 }
 
-// nb = sqrt(q) and g = 1 / (q + al nb) of a normal q > 0, al >= 0, to rounding.
+// nb = sqrt(q) and g = 1 / (q + al nb) for al >= 0, al^2 <= q and 2^-959 <= q <=
+// 2^960, to rounding (errors < 1.55 and 3 times 2^-53; outside, y or r may be 0
+// or infinite and the result NaN: warp_qr_panel_scaled).
 // y ~ 1 / sqrt(q) and r ~ 1 / (q + al sqrt(q)) are the hardware's
 // approximations (2^-20), each corrected by one third-order Newton step:
 // with t = q y, e = 1 - t y:  sqrt(q) = t (1 + e / 2 + 3 e^2 / 8 + O(e^3)), and
@@ -57,6 +61,9 @@ __device__ __forceinline__ void sqrt_rcp(double q, double al, double &nb, double
   const double f = fma(-fma(al, nb, q), r, 1.0);
   g = fma(r, fma(f, f, f), r);
 }
+
+// The exponent field of x (x = m 2^(exp_of - 1023), 1 <= m < 2).
+__device__ __forceinline__ unsigned exp_of(double x) { return ((unsigned)__double2hiint(x) >> 20) & 0x7ffu; }
 
 // An 8 x 8 accumulator (row lane / 4, columns 2 (lane % 4) + {0, 1}) as the two
 // B fragments of a product over its rows: b[s] = X(4 s + lane % 4, lane / 4).
@@ -151,9 +158,13 @@ __device__ __forceinline__ void panel_update(double *A, int lda, int n, int j0, 
 // (zeros above) into Vb (column c at c ldv), and the block's T (DLARFT forward /
 // columnwise with g for tau, column-major 8 x 8) into Tb; the products
 // v_q^T v_k it needs come with the same sums, through the 64 doubles zs.
+// Returns false with nothing written (unless any) where a diagonal entry of R is
+// outside [2^-100, 2^100) (or NaN: the squares left the range): then squares, or
+// products of an unscaled reflector with a column, may over- or underflow.
+// (Scaling a column at its step, in the column's chain, cost 1 to 3 % of a bin.)
 template <int R>
-__device__ __forceinline__ void warp_qr_panel(double *A, int lda, int n, int j0, double *Vb, int ldv,
-                                              double *Tb, double *vd, double *zs) {
+__device__ __forceinline__ bool warp_qr_panel(double *A, int lda, int n, int j0, double *Vb, int ldv,
+                                              double *Tb, double *vd, double *zs, bool any) {
   const int lane = threadIdx.x & 31, lr = lane >> 2, lc = lane & 3;
   const int mp = n - j0, ib = mp < WY_NB ? mp : WY_NB;
   double *Ap = A + j0 + (j0 + 2 * lc) * lda + lr;
@@ -217,6 +228,10 @@ __device__ __forceinline__ void warp_qr_panel(double *A, int lda, int n, int j0,
     column(k, WyIdx<0>{});
     if (k + 1 < ib) column(k + 1, WyIdx<1>{});
   }
+  // row r's lane of column r: R(r, r), the column's norm at its step
+  const double rr = (lr & 1) ? a[0][1] : a[0][0];
+  const bool far = (lr >> 1) == lc && lr < ib && exp_of(rr) - 923u >= 200u;
+  if (__any_sync(Z2_FULL, far) && !any) return false;
   for (int t = 8 * ib + lane; t < 64; t += 32) zs[t] = 0.0;   // columns past the matrix
   __syncwarp();
   const int m8 = (mp + 7) & ~7;
@@ -253,25 +268,57 @@ __device__ __forceinline__ void warp_qr_panel(double *A, int lda, int n, int j0,
     for (int c = 0; c < 8; ++c) Tb[c * 8 + lane] = tr[c];
   }
   __syncwarp();
+  return true;
 }
 
 // The panel with the smallest R that holds its n - j0 <= 32 T rows.
 template <bool SH, int T>
-__device__ __noinline__ void warp_qr_panel_any(double *A, int lda, int n, int j0, double *Vb, int ldv,
-                                               double *Tb, double *vd, double *zs) {
+__device__ __noinline__ bool warp_qr_panel_any(double *A, int lda, int n, int j0, double *Vb, int ldv,
+                                               double *Tb, double *vd, double *zs, bool any) {
   if (SH) A = as_shared(A);
   zs = as_shared(zs);
   Vb = as_shared(Vb);
   Tb = as_shared(Tb);
   vd = as_shared(vd);
   const int mp = n - j0;
-  if (T > 5 && mp > 160) warp_qr_panel<32>(A, lda, n, j0, Vb, ldv, Tb, vd, zs);
-  else if (T > 4 && mp > 144) warp_qr_panel<20>(A, lda, n, j0, Vb, ldv, Tb, vd, zs);
-  else if (T > 3 && mp > 104) warp_qr_panel<18>(A, lda, n, j0, Vb, ldv, Tb, vd, zs);
-  else if (T > 2 && mp > 64) warp_qr_panel<13>(A, lda, n, j0, Vb, ldv, Tb, vd, zs);
-  else if (T > 1 && mp > 32) warp_qr_panel<8>(A, lda, n, j0, Vb, ldv, Tb, vd, zs);
-  else if (mp > 16) warp_qr_panel<4>(A, lda, n, j0, Vb, ldv, Tb, vd, zs);
-  else warp_qr_panel<2>(A, lda, n, j0, Vb, ldv, Tb, vd, zs);
+  if (T > 5 && mp > 160) return warp_qr_panel<32>(A, lda, n, j0, Vb, ldv, Tb, vd, zs, any);
+  if (T > 4 && mp > 144) return warp_qr_panel<20>(A, lda, n, j0, Vb, ldv, Tb, vd, zs, any);
+  if (T > 3 && mp > 104) return warp_qr_panel<18>(A, lda, n, j0, Vb, ldv, Tb, vd, zs, any);
+  if (T > 2 && mp > 64) return warp_qr_panel<13>(A, lda, n, j0, Vb, ldv, Tb, vd, zs, any);
+  if (T > 1 && mp > 32) return warp_qr_panel<8>(A, lda, n, j0, Vb, ldv, Tb, vd, zs, any);
+  if (mp > 16) return warp_qr_panel<4>(A, lda, n, j0, Vb, ldv, Tb, vd, zs, any);
+  return warp_qr_panel<2>(A, lda, n, j0, Vb, ldv, Tb, vd, zs, any);
+}
+
+// Panel j0 by one warp; where the plain one gives up, on scaled columns: every
+// column of the panel times a power of two that brings its largest entry into
+// [1, 2).  The reflectors, v(j) and g of the scaled columns give the same H; R is
+// scaled back.  Lane l looks after column l / 4, rows l % 4 + 4 i.
+template <bool SH, int T>
+__device__ __noinline__ void warp_qr_panel_scaled(double *A, int lda, int n, int j0, double *Vb, int ldv,
+                                                  double *Tb, double *vd, double *zs) {
+  const int lane = threadIdx.x & 31, c = lane >> 2, r0 = lane & 3, mp = n - j0;
+  double *Ac = A + j0 + (j0 + c) * lda;
+  const int m = c < mp ? mp : 0;
+  double mx = 0.0, un = 1.0;
+  for (int r = r0; r < m; r += 4) mx = fmax(mx, fabs(Ac[r]));
+  mx = fmax(mx, __shfl_xor_sync(Z2_FULL, mx, 1));
+  mx = fmax(mx, __shfl_xor_sync(Z2_FULL, mx, 2));
+  if (mx > 0.0) {
+    const int b = min(max(2046 - (int)exp_of(mx), 1), 2045);      // times 2^(b - 1023)
+    for (int r = r0; r < m; r += 4) Ac[r] *= __hiloint2double(b << 20, 0);
+    un = __hiloint2double((2046 - b) << 20, 0);
+  }
+  __syncwarp();
+  warp_qr_panel_any<SH, T>(A, lda, n, j0, Vb, ldv, Tb, vd, zs, true);
+  for (int r = r0; r < min(c + 1, m); r += 4) Ac[r] *= un;
+  __syncwarp();
+}
+template <bool SH, int T>
+__device__ __forceinline__ void warp_qr_panel_safe(double *A, int lda, int n, int j0, double *Vb, int ldv,
+                                                   double *Tb, double *vd, double *zs) {
+  if (!warp_qr_panel_any<SH, T>(A, lda, n, j0, Vb, ldv, Tb, vd, zs, false))
+    warp_qr_panel_scaled<SH, T>(A, lda, n, j0, Vb, ldv, Tb, vd, zs);
 }
 
 // C <- C - V (op(T) (V^T C)) for NT tiles of 8 columns of A, rows j0..n, by one
@@ -356,7 +403,7 @@ __device__ __noinline__ void blk_qr_panels(double *A, int lda, int n, double *vd
   const int warp = threadIdx.x >> 5;
   const int ldv = wy_ldv(n), np = wy_panels(n);
   double *Tall = work + 2 * WY_NB * ldv, *zs = Tall + 64 * np;
-  if (warp == 0) warp_qr_panel_any<SH, T>(A, lda, n, 0, work, ldv, Tall, vd, zs);
+  if (warp == 0) warp_qr_panel_safe<SH, T>(A, lda, n, 0, work, ldv, Tall, vd, zs);
   __syncthreads();
   for (int p = 0; p + 1 < np; ++p) {
     const int j0 = p * WY_NB;
@@ -364,8 +411,8 @@ __device__ __noinline__ void blk_qr_panels(double *A, int lda, int n, double *vd
     // warp 0: the next panel's tile, then that panel; the others the rest
     wy_tiles<true>(A, lda, n, j0, p + 1 + warp, warp == 0 ? np : Z2_WARPS - 1, np, Vb, ldv, Tb);
     if (warp == 0)
-      warp_qr_panel_any<SH, T>(A, lda, n, j0 + WY_NB, work + ((p + 1) & 1) * WY_NB * ldv, ldv,
-                               Tall + (p + 1) * 64, vd, zs);
+      warp_qr_panel_safe<SH, T>(A, lda, n, j0 + WY_NB, work + ((p + 1) & 1) * WY_NB * ldv, ldv,
+                                Tall + (p + 1) * 64, vd, zs);
     __syncthreads();
   }
 }
