@@ -388,8 +388,11 @@ extern "C" int z2_create(z2_handle **out, const z2_chain_params *params, int32_t
     if (C.d.g_in_smem && nn + std::max<size_t>(2 * (size_t)z2_ldx(N) * C.d.k2, tile_min(N)) > arena)
       C.d.g_in_smem = 0;
   }
+  // the limit belongs to the function, not to the handle: always the largest, so
+  // that a later handle does not lower it under an earlier one (a launch takes
+  // what it asks for)
   CUDA_TRY(h, cudaFuncSetAttribute(z2_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)h->smem));
+                                   kSmemMax));
   CUDA_TRY(h, cudaMalloc(&h->d_status, sizeof(int) * nchains));
   CUDA_TRY(h, cudaMemset(h->d_status, 0, sizeof(int) * nchains));
   h->h_status.assign(nchains, 0);
@@ -588,7 +591,7 @@ extern "C" int z2_create(z2_handle **out, const z2_chain_params *params, int32_t
   for (const auto &C : h->ch) nmax = std::max(nmax, C.N);
   h->small_blocks = nmax <= 64 && nchains > nsm && !h->opt.stab_exact;
   if (h->small_blocks) {
-    CUDA_TRY(h, z2_small_setup((int)h->smem, &occ));
+    CUDA_TRY(h, z2_small_setup(kSmemMax, h->smem, &occ));
     occ = small_blocks_per_sm(*h, nsm, occ);
   } else {
     CUDA_TRY(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, z2_chain_kernel, Z2_NT, h->smem));

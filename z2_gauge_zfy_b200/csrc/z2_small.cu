@@ -12,8 +12,8 @@ namespace z2w4 {
 }
 #include "z2_small.h"
 
-cudaError_t z2_small_setup(int smem, int *blocks) {
-  cudaError_t e = cudaFuncSetAttribute(z2w4::z2_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+cudaError_t z2_small_setup(int limit, unsigned smem, int *blocks) {
+  cudaError_t e = cudaFuncSetAttribute(z2w4::z2_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
   if (e != cudaSuccess) return e;
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, z2w4::z2_chain_kernel, Z2_NT, smem);
 }

@@ -3,8 +3,9 @@
 #pragma once
 #include <cuda_runtime.h>
 
-// Sets the kernel up for smem bytes per block; *blocks: resident blocks per SM.
-cudaError_t z2_small_setup(int smem, int *blocks);
+// Allows launches of up to limit bytes of dynamic shared memory; *blocks: resident
+// blocks per SM at smem bytes.
+cudaError_t z2_small_setup(int limit, unsigned smem, int *blocks);
 // One launch; descs is a device array of ChainDesc, op one of OP_PRE, OP_SWEEP,
 // OP_GLOBAL, OP_THERM.
 cudaError_t z2_small_launch(int grid, unsigned smem, cudaStream_t stream, const void *descs, const int *order,
