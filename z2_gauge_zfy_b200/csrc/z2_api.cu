@@ -7,9 +7,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
-#include <functional>
 #include <initializer_list>
-#include <queue>
 #include <string>
 #include <vector>
 
@@ -18,6 +16,7 @@ namespace z2w8 {
 #include "z2_kernel.cuh"
 }
 using namespace z2w8;
+#include "z2_schedule.h"
 #include "z2_small.h"
 
 static_assert(PH_COUNT == Z2_NPHASE, "phase counters and the C ABI disagree");
@@ -184,42 +183,7 @@ struct z2_handle {
   size_t u_n = 0;
 };
 
-// Relative time of one chain's bin, from the cycles per slice measured at N = 16,
-// 36, 64, 100, 144 (65, 134, 183, 466, 688 K) and 256 (5 M: G outside the SM).
-static double chain_cost(const ChainHost &C) {
-  const double n = C.N;
-  return (double)C.Ltrot * (30.0 + 2.2 * n + 0.016 * n * n) * (C.d.g_in_smem ? 1.0 : 3.0);
-}
-
-// Blocks per SM of the 128-thread kernel: the count with the shortest schedule of
-// the work queue (longest chain first onto the first free block), given how
-// much a chain slows down beside others on its SM.  Measured on 6 x 6 lattices,
-// 40 slices (ms per round of b blocks per SM): 2.4, 3.1, 3.9, 4.9 for b = 1..4;
-// throughput is level from b = 2 (2000 chains: 39, 28, 28, 28 ms), so b rises
-// above 2 where it saves a round (300 8 x 8 chains: 8.8 ms at 2, 5.9 at 3) and
-// stays at 2 where a few long chains set the time (512 chains of 4 x 4 and
-// 6 x 6: 7.9 ms at 2, 10.1 at 4; one 256-thread block per SM: 9.8).
-static int small_blocks_per_sm(const z2_handle &h, int nsm, int occ) {
-  static const double slow[5] = {1.0, 1.0, 1.3, 1.65, 2.05};
-  std::vector<double> cost;
-  for (const auto &C : h.ch) cost.push_back(chain_cost(C));
-  std::sort(cost.begin(), cost.end(), std::greater<double>());
-  int best = 1;
-  double tbest = 0.0;
-  for (int b = 1; b <= std::min(occ, 4); ++b) {
-    std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
-    for (int i = 0; i < b * nsm; ++i) free_at.push(0.0);
-    double t = 0.0;
-    for (double x : cost) {
-      const double end = free_at.top() + x * slow[b];
-      free_at.pop();
-      free_at.push(end);
-      t = std::max(t, end);
-    }
-    if (b == 1 || t < tbest) { best = b; tbest = t; }
-  }
-  return best;
-}
+static double chain_cost(const ChainHost &C) { return z2_chain_cost(C.N, C.Ltrot, C.d.g_in_smem != 0); }
 
 static int set_err(z2_handle *h, int code, const char *fmt, ...) {
   if (h) {
@@ -585,15 +549,19 @@ extern "C" int z2_create(z2_handle **out, const z2_chain_params *params, int32_t
   int nsm = 0, occ = 0;
   CUDA_TRY(h, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device));
   // Lattices of up to 64 sites, more chains than SMs: 128-thread blocks, several
-  // per SM (a chain alone runs slower on them, so with an SM per chain the
-  // 256-thread block stays).  The reference's pivoted QR needs 256 threads.
+  // per SM, where their schedule is the shorter one (z2_schedule.h).  The
+  // reference's pivoted QR needs 256 threads.
   int nmax = 0;
   for (const auto &C : h->ch) nmax = std::max(nmax, C.N);
   h->small_blocks = nmax <= 64 && nchains > nsm && !h->opt.stab_exact;
   if (h->small_blocks) {
     CUDA_TRY(h, z2_small_setup(kSmemMax, h->smem, &occ));
-    occ = small_blocks_per_sm(*h, nsm, occ);
-  } else {
+    std::vector<Z2ChainLoad> load;
+    for (const auto &C : h->ch) load.push_back({C.N, chain_cost(C)});
+    occ = z2_small_blocks_per_sm(load, nsm, occ);
+    h->small_blocks = occ > 0;
+  }
+  if (!h->small_blocks) {
     CUDA_TRY(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, z2_chain_kernel, Z2_NT, h->smem));
   }
   if (occ < 1) occ = 1;

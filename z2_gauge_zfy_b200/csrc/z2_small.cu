@@ -2,7 +2,7 @@
 // registers per thread (compiled with -maxrregcount=128): four blocks share an
 // SM's register file where the 256-thread build fills it with one.  For
 // launches of more chains than SMs on lattices of up to 64 sites, whose chains
-// are bound by latency and leave most of an SM idle (the rule is in z2_create).
+// are bound by latency and leave most of an SM idle (the rule is in z2_schedule.h).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
