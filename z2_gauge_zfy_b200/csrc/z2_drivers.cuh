@@ -314,13 +314,13 @@ __device__ __noinline__ void chain_therm(const ChainDesc &c, const Smem &s, int 
         const signed char *sp = sig + (size_t)((t - 1 + L) % L) * nb;
         const signed char *sn = sig + (size_t)((t + 1) % L) * nb;
         for (int b = 0; b < nb; ++b) {
-          const int *bb = c.bbonds + 6 * b;
-          const double s_old = (double)sg[b];
-          const double tmp_old = s_old * sg[bb[0]] * sg[bb[1]] * sg[bb[2]] +
-                                 s_old * sg[bb[3]] * sg[bb[4]] * sg[bb[5]];
-          const int is = (int)(-2.0 * tmp_old + 4.0) >> 2;
-          const double tn = s_old * ((double)sp[b] + (double)sn[b]);
-          const int it = (int)(-2.0 * tn + 4.0) >> 2;
+          // the two plaquettes' and the neighbours' signs pick the entry of the table
+          const int2 *bb = reinterpret_cast<const int2 *>(c.bbonds) + 3 * b;
+          const int2 u = bb[0], v = bb[1], w2 = bb[2];
+          const int s_old = sg[b];
+          const int x = s_old ^ sg[u.x] ^ sg[u.y] ^ sg[v.x], y = s_old ^ sg[v.y] ^ sg[w2.x] ^ sg[w2.y];
+          const int is = (x < 0) + (y < 0);
+          const int it = 1 - ((s_old * (sp[b] + sn[b])) >> 1);
           st = ranf_next(st);
           if (c.rb[is * 3 + it] > (double)st * (1.0 / 2147483648.0)) {
             sg[b] = (signed char)(-sg[b]);
