@@ -19,7 +19,9 @@ UNITS = (("z2_api.cu", []), ("z2_small.cu", ["-maxrregcount=128"]))
 OUT = os.path.join(HERE, "libz2dqmc.so")
 # Relocatable device code: ptxas optimises a whole program's call graph at
 # once, and for this one that took over ten minutes; function by function it
-# takes half a minute.
+# takes half a minute.  The device functions are static, so that the compiler
+# still sees all their callers (address spaces, constants): with external linkage
+# the time-displaced correlators took a quarter longer.
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = [*ARCH, "-O3", "-lineinfo", "-std=c++17", "-dc", "-Xcompiler", "-fPIC"]
 

@@ -273,7 +273,7 @@ __device__ __forceinline__ bool warp_qr_panel(double *A, int lda, int n, int j0,
 
 // The panel with the smallest R that holds its n - j0 <= 32 T rows.
 template <bool SH, int T>
-__device__ __noinline__ bool warp_qr_panel_any(double *A, int lda, int n, int j0, double *Vb, int ldv,
+static __device__ __noinline__ bool warp_qr_panel_any(double *A, int lda, int n, int j0, double *Vb, int ldv,
                                                double *Tb, double *vd, double *zs, bool any) {
   if (SH) A = as_shared(A);
   zs = as_shared(zs);
@@ -295,7 +295,7 @@ __device__ __noinline__ bool warp_qr_panel_any(double *A, int lda, int n, int j0
 // [1, 2).  The reflectors, v(j) and g of the scaled columns give the same H; R is
 // scaled back.  Lane l looks after column l / 4, rows l % 4 + 4 i.
 template <bool SH, int T>
-__device__ __noinline__ void warp_qr_panel_scaled(double *A, int lda, int n, int j0, double *Vb, int ldv,
+static __device__ __noinline__ void warp_qr_panel_scaled(double *A, int lda, int n, int j0, double *Vb, int ldv,
                                                   double *Tb, double *vd, double *zs) {
   const int lane = threadIdx.x & 31, c = lane >> 2, r0 = lane & 3, mp = n - j0;
   double *Ac = A + j0 + (j0 + c) * lda;
@@ -397,7 +397,7 @@ __device__ __forceinline__ void wy_tiles(double *A, int lda, int n, int j0, int 
 // reflectors in A, their diagonals in vd (n doubles of shared memory), every
 // panel's T in work (wy_work(n) doubles of it): what blk_form_q takes.
 template <bool SH, int T>
-__device__ __noinline__ void blk_qr_panels(double *A, int lda, int n, double *vd, double *work) {
+static __device__ __noinline__ void blk_qr_panels(double *A, int lda, int n, double *vd, double *work) {
   if (SH) A = as_shared(A);
   work = as_shared(work);
   const int warp = threadIdx.x >> 5;
@@ -421,7 +421,7 @@ __device__ __noinline__ void blk_qr_panels(double *A, int lda, int n, double *vd
 // coefficients tau): one panel per warp, S = V^T V by DMMA, T by the recurrence
 // of warp_qr_panel; vd = 1.
 template <bool SH>
-__device__ __noinline__ void blk_wy_t(const double *A, int lda, int n, const double *tau, double *vd,
+static __device__ __noinline__ void blk_wy_t(const double *A, int lda, int n, const double *tau, double *vd,
                                       double *work) {
   if (SH) A = as_shared(const_cast<double *>(A));
   double *Tall = as_shared(work) + 2 * WY_NB * wy_ldv(n);
@@ -485,7 +485,7 @@ __device__ __forceinline__ void wy_load_v(double *A, int lda, int n, int p, cons
 // next panel's reflectors are taken out of A while the current one is
 // applied: one block barrier per panel.
 template <bool SH>
-__device__ __noinline__ void blk_form_q(double *A, int lda, int n, const double *vd, double *work) {
+static __device__ __noinline__ void blk_form_q(double *A, int lda, int n, const double *vd, double *work) {
   if (SH) A = as_shared(A);
   work = as_shared(work);
   const int warp = threadIdx.x >> 5;
@@ -659,7 +659,7 @@ __device__ __forceinline__ void gj_tiles(double *M, int ldm, int n, int first, i
 //   M^-1(j, piv[m]) = (M on exit)(piv[j], m).
 // work: 2 WY_NB wy_ldv(n) doubles of shared memory, piv n ints of it.
 template <bool SH, int T>
-__device__ __noinline__ void blk_gj_panels(double *M, int ldm, int n, int *piv, double *work) {
+static __device__ __noinline__ void blk_gj_panels(double *M, int ldm, int n, int *piv, double *work) {
   if (SH) M = as_shared(M);
   work = as_shared(work);
   piv = as_shared(piv);

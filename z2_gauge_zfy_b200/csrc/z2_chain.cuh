@@ -18,7 +18,7 @@
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 
-__device__ Smem make_smem(const ChainDesc &c, unsigned char *base, size_t smem_bytes) {
+static __device__ Smem make_smem(const ChainDesc &c, unsigned char *base, size_t smem_bytes) {
   Smem s;
   const int N = c.N;
   size_t off = 0;
@@ -57,7 +57,7 @@ __device__ Smem make_smem(const ChainDesc &c, unsigned char *base, size_t smem_b
 // src/multiply.f90:106).  L chain (ULT = UL^T, B symmetric): for nt' = hi
 // down to lo, ULT *= e^{dtau mu} then ULT <- B_nt' ULT (propT_L + prop_L,
 // src/multiply.f90:91, src/localK.f90:370).
-__device__ __noinline__ void pending_mu(const ChainDesc &c, double *A, int lda, int n) {
+static __device__ __noinline__ void pending_mu(const ChainDesc &c, double *A, int lda, int n) {
   if (c.eP == 1.0) return;
   double x = 1.0;
   for (int i = 0; i < n; ++i) x *= c.eP;       // one pass for the n slices' factors
@@ -91,7 +91,7 @@ __device__ __forceinline__ void apply_pending_L(const ChainDesc &c, const Smem &
 // N x N x N products (at N = 100, 0.5 M cycles against 9 M for the 2N x 2N QR).
 // M (ldm): work matrix (shared arena when it fits); W0..W3 N x N global
 // workspaces; outputs N x N (ld N).
-__device__ __noinline__ void dev_stab_green_big(const Smem &s, int N, const double *UR, const double *DR,
+static __device__ __noinline__ void dev_stab_green_big(const Smem &s, int N, const double *UR, const double *DR,
                                    const double *VR, const double *ULT, const double *DL,
                                    const double *VL, double *M, int ldm, double *W0, double *W1,
                                    double *W2, double *W3, double *G00, double *G0t, double *Gt0,
@@ -142,7 +142,7 @@ __device__ __noinline__ void dev_stab_green_big(const Smem &s, int N, const doub
 // pass over all (i, j) with a gather of the phase took 20 K cycles per slice at
 // N = 144.)
 template <bool GS>
-__device__ __noinline__ void obs_equal_on(const ChainDesc &c, const Smem &s, int nt) {
+static __device__ __noinline__ void obs_equal_on(const ChainDesc &c, const Smem &s, int nt) {
   const int N = c.N, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const double *G = GS ? as_shared(s.G) : s.G;
   const int ldg = s.ldg;
@@ -211,7 +211,7 @@ __device__ __forceinline__ void obs_equal(const ChainDesc &c, const Smem &s, int
 // parts, both identical spin sectors summed; binned by imj deterministically
 // (one thread per displacement).
 // ---------------------------------------------------------------------------
-__device__ __noinline__ void obs_tau(const ChainDesc &c, const Smem &s, int nt) {
+static __device__ __noinline__ void obs_tau(const ChainDesc &c, const Smem &s, int nt) {
   const int N = c.N, Lx = c.Lx, Ly = c.Ly;
   const double *G00 = c.G00, *Gtt = c.Gtt, *Gt0 = c.Gt0, *G0t = c.G0t;
   const signed char *sgt = c.sigma + (size_t)(nt - 1) * c.nb;
@@ -281,10 +281,10 @@ __device__ __forceinline__ double *qr_matrix(const ChainDesc &c, const Smem &s, 
   return s.Wq;
 }
 
-__device__ __noinline__ void spill_G(const ChainDesc &c, const Smem &s) {
+static __device__ __noinline__ void spill_G(const ChainDesc &c, const Smem &s) {
   if (c.g_in_smem) blk_copy(c.G, c.N, s.G, s.ldg, c.N, c.N);
 }
-__device__ __noinline__ void load_G(const ChainDesc &c, const Smem &s) {
+static __device__ __noinline__ void load_G(const ChainDesc &c, const Smem &s) {
   if (c.g_in_smem) blk_copy(s.G, s.ldg, c.G, c.N, c.N, c.N);
 }
 
@@ -292,7 +292,7 @@ __device__ __noinline__ void load_G(const ChainDesc &c, const Smem &s) {
 // over both: returns the drift max |Gn - G| (compare_mat,
 // src/stabilization.f90:365-372) and leaves G = Gn in global memory and, for
 // a chain whose G lives in shared memory, there too.
-__device__ __noinline__ double take_green(const ChainDesc &c, const Smem &s, const double *Gn) {
+static __device__ __noinline__ double take_green(const ChainDesc &c, const Smem &s, const double *Gn) {
   const int N = c.N, ldg = s.ldg;
   double *Gg = c.G, *Gs = s.G;
   const bool sm = c.g_in_smem != 0;
@@ -310,12 +310,12 @@ __device__ __noinline__ double take_green(const ChainDesc &c, const Smem &s, con
   return r;
 }
 
-__device__ __noinline__ void copy_vec(double *dst, const double *src, int n) {
+static __device__ __noinline__ void copy_vec(double *dst, const double *src, int n) {
   for (int i = threadIdx.x; i < n; i += Z2_NT) dst[i] = src[i];
   __syncthreads();
 }
 
-__device__ __noinline__ void record_drift(const ChainDesc &c, double dif, bool stats) {
+static __device__ __noinline__ void record_drift(const ChainDesc &c, double dif, bool stats) {
   if (threadIdx.x == 0) {
     if (dif > c.acc[A_XMAX] || dif != dif) c.acc[A_XMAX] = dif;
     if (stats) c.acc[A_XMEAN] += dif;
@@ -341,7 +341,7 @@ __device__ __forceinline__ void chain_stab_green(const ChainDesc &c, const Smem 
 }
 
 // Wrap_pre (src/stabilization.f90:374-398)
-__device__ __noinline__ void wrap_pre(const ChainDesc &c, const Smem &s, int nt, Pend &pd) {
+static __device__ __noinline__ void wrap_pre(const ChainDesc &c, const Smem &s, int nt, Pend &pd) {
   const int N = c.N, NN = N * N;
   int lda; double *A = qr_matrix(c, s, lda);
   const int st = nt / c.Nwrap;
@@ -361,7 +361,7 @@ __device__ __noinline__ void wrap_pre(const ChainDesc &c, const Smem &s, int nt,
 }
 
 // Wrap_L (src/stabilization.f90:400-437)
-__device__ __noinline__ void wrap_L(const ChainDesc &c, const Smem &s, int nt, Pend &pd, bool stats) {
+static __device__ __noinline__ void wrap_L(const ChainDesc &c, const Smem &s, int nt, Pend &pd, bool stats) {
   const int N = c.N, NN = N * N;
   spill_G(c, s);
   int lda; double *A = qr_matrix(c, s, lda);
@@ -391,7 +391,7 @@ __device__ __noinline__ void wrap_L(const ChainDesc &c, const Smem &s, int nt, P
 }
 
 // Wrap_R (src/stabilization.f90:439-476)
-__device__ __noinline__ void wrap_R(const ChainDesc &c, const Smem &s, int nt, Pend &pd, bool stats) {
+static __device__ __noinline__ void wrap_R(const ChainDesc &c, const Smem &s, int nt, Pend &pd, bool stats) {
   const int N = c.N, NN = N * N;
   spill_G(c, s);
   int lda; double *A = qr_matrix(c, s, lda);

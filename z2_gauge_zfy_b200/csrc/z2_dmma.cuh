@@ -37,7 +37,7 @@ struct MatRef {
 // groups of 8 x 8 DMMA tiles; interior groups run a pointer-increment loop
 // without bounds checks.  beta == 0 never reads C.  Ends with the block
 // synchronised.
-__device__ __noinline__ void blk_dmma(int m, int n, int k, double alpha, MatRef A, bool a_upper,
+static __device__ __noinline__ void blk_dmma(int m, int n, int k, double alpha, MatRef A, bool a_upper,
                                      MatRef B, bool b_lower, double beta, double *C, int ldc) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int lr = lane >> 2, lc = lane & 3;
@@ -205,7 +205,7 @@ __device__ __forceinline__ double sumsq_col(const double *x, int i0, int n) {
 
 // Pivoted Householder QR, DGEQP3/DLAQP2 semantics (all columns free), with the
 // trailing update and the norm downdate done one thread per column.
-__device__ __noinline__ void blk_geqp3_tc(double *A, int lda, int n, int *jpvt, double *tau,
+static __device__ __noinline__ void blk_geqp3_tc(double *A, int lda, int n, int *jpvt, double *tau,
                                          double *vn1, double *vn2) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const double tol3z = 1.0536712127723509e-08;   // sqrt(dlamch('E'))
@@ -281,7 +281,7 @@ __device__ __noinline__ void blk_geqp3_tc(double *A, int lda, int n, int *jpvt, 
 }
 
 // DORG2R (m x n, n reflectors) with one thread per trailing column.
-__device__ __noinline__ void blk_org2r_tc(double *A, int lda, int m, int n, const double *tau) {
+static __device__ __noinline__ void blk_org2r_tc(double *A, int lda, int m, int n, const double *tau) {
   for (int i = n - 1; i >= 0; --i) {
     const double ti = tau[i];
     const double *v = A + (size_t)i * lda;
@@ -308,7 +308,7 @@ __device__ __noinline__ void blk_org2r_tc(double *A, int lda, int m, int n, cons
 // Solve L Z = Y in place, L unit lower triangular (below the diagonal of L),
 // Y n x nc: blocks of 8 rows from the top, the 8 x 8 diagonal block solved one
 // thread per column in registers, the rows below updated by DMMA.
-__device__ __noinline__ void blk_trsm_lln_blocked(const double *L, int ldl, int n, double *Y,
+static __device__ __noinline__ void blk_trsm_lln_blocked(const double *L, int ldl, int n, double *Y,
                                                   int ldy, int nc) {
   for (int k0 = 0; k0 < n; k0 += 8) {
     const int kb = (n - k0) < 8 ? (n - k0) : 8;
@@ -341,7 +341,7 @@ __device__ __noinline__ void blk_trsm_lln_blocked(const double *L, int ldl, int 
   }
 }
 
-__device__ __noinline__ void blk_trsm_lun_blocked(const double *R, int ldr, int n, double *Y,
+static __device__ __noinline__ void blk_trsm_lun_blocked(const double *R, int ldr, int n, double *Y,
                                                   int ldy, int nc);
 
 // Inverse of a general n x n matrix by LU with partial pivoting (the
@@ -352,7 +352,7 @@ __device__ __noinline__ void blk_trsm_lun_blocked(const double *R, int ldr, int 
 // A^-1 = U^-1 L^-1 P from the identity by the two blocked triangular solves.
 // A is overwritten by its inverse; W (ldw) is an n x n workspace; work holds
 // 256 doubles of shared memory.
-__device__ __noinline__ void blk_inverse_blocked(double *A, int lda, int n, double *W, int ldw,
+static __device__ __noinline__ void blk_inverse_blocked(double *A, int lda, int n, double *W, int ldw,
                                                  int *ipiv, double *red, int *flag, double *work) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int j0 = 0; j0 < n; j0 += 16) {
@@ -444,7 +444,7 @@ __device__ __noinline__ void blk_inverse_blocked(double *A, int lda, int n, doub
 // (ldr).  Blocks of 8 rows from the bottom: the 8 x 8 diagonal block is
 // solved one thread per column (block of R held in registers), the rows
 // above are updated by DMMA.
-__device__ __noinline__ void blk_trsm_lun_blocked(const double *R, int ldr, int n, double *Y,
+static __device__ __noinline__ void blk_trsm_lun_blocked(const double *R, int ldr, int n, double *Y,
                                                   int ldy, int nc) {
   const int last = ((n - 1) / 8) * 8;
   for (int k0 = last; k0 >= 0; k0 -= 8) {

@@ -4,7 +4,7 @@
 #include "z2_chain.cuh"
 
 // Wrap_tau (src/stabilization.f90:478-514) on the Dyn copy of the propagator.
-__device__ __noinline__ void wrap_tau(const ChainDesc &c, const Smem &s, int nt, Pend &pd) {
+static __device__ __noinline__ void wrap_tau(const ChainDesc &c, const Smem &s, int nt, Pend &pd) {
   const int N = c.N, NN = N * N;
   int lda; double *A = qr_matrix(c, s, lda);
   const int st = nt / c.Nwrap;
@@ -47,7 +47,7 @@ __device__ __noinline__ void wrap_tau(const ChainDesc &c, const Smem &s, int nt,
 // Dyn_reset (src/dynamics.f90:41-48, Propgr_reset src/process_matrix.f90:88-96):
 // the Dyn copy of the propagator and G00 = Gtt = Gt0 = G, G0t = -(I - G),
 // from the chain's G in global memory.
-__device__ __noinline__ void dyn_reset(const ChainDesc &c, const Smem &s) {
+static __device__ __noinline__ void dyn_reset(const ChainDesc &c, const Smem &s) {
   const int N = c.N;
   blk_copy(c.URd, N, c.UR, N, N, N);
   blk_copy(c.VRd, N, c.VR, N, N, N);
@@ -70,7 +70,7 @@ __device__ __noinline__ void dyn_reset(const ChainDesc &c, const Smem &s) {
 // propgrK_R (src/multiply.f90:43-63) without the U factor, and propgrT_R
 // (src/multiply.f90:110-130): Gt0 <- B Gt0, G0t <- G0t B^-1, Gtt <- B Gtt B^-1,
 // then the mu factors.
-__device__ __noinline__ void propgr_R(const ChainDesc &c, const Smem &s, int nt, bool kin, bool mu) {
+static __device__ __noinline__ void propgr_R(const ChainDesc &c, const Smem &s, int nt, bool kin, bool mu) {
   const int N = c.N;
   if (kin && c.use_kin) {
     build_table(c, s, nt);
@@ -88,7 +88,7 @@ __device__ __noinline__ void propgr_R(const ChainDesc &c, const Smem &s, int nt,
 
 // Dyn_reset + Dyn_sweep_R (src/dynamics.f90:41-62): the G(tau,0) chain.
 // The arena is free here (G is spilled in c.G).
-__device__ __noinline__ void dyn_sweep(const ChainDesc &c, const Smem &s) {
+static __device__ __noinline__ void dyn_sweep(const ChainDesc &c, const Smem &s) {
   dyn_reset(c, s);
   Pend pd{1, 0};
   for (int nt = 1; nt <= c.Ltrot; ++nt) {
@@ -100,7 +100,7 @@ __device__ __noinline__ void dyn_sweep(const ChainDesc &c, const Smem &s) {
 }
 
 // Local_sweep_pre (src/local_sweep.f90:87-104)
-__device__ __noinline__ void chain_pre(const ChainDesc &c, const Smem &s) {
+static __device__ __noinline__ void chain_pre(const ChainDesc &c, const Smem &s) {
   const int N = c.N;
   if (threadIdx.x == 0) c.acc[A_NOTBETA] = 0.0;   // is_beta = .true. (src/main.f90:73)
   if (c.hzero) {   // this%reset (src/local_sweep.f90:63-69): sigma constant in tau
@@ -121,7 +121,7 @@ __device__ __noinline__ void chain_pre(const ChainDesc &c, const Smem &s) {
   }
 }
 
-__device__ __noinline__ void scale_G_mu(const ChainDesc &c, const Smem &s) {
+static __device__ __noinline__ void scale_G_mu(const ChainDesc &c, const Smem &s) {
   if (c.eP != 1.0 || c.eM != 1.0) {
     blk_scale(s.G, s.ldg, c.N, c.N, c.eP);
     blk_scale(s.G, s.ldg, c.N, c.N, c.eM);
@@ -141,7 +141,7 @@ __device__ __forceinline__ void l2_prefetch(const double *p, int n) {
 // slice ahead of it: the stack entry st of the other sweep direction (kept
 // since the previous sweep) and this direction's U, V, D (from the previous
 // wrap), which other chains' traffic has usually evicted by then.
-__device__ __noinline__ void prefetch_wrap(const ChainDesc &c, int st, bool left) {
+static __device__ __noinline__ void prefetch_wrap(const ChainDesc &c, int st, bool left) {
   const int N = c.N, NN = N * N;
   if (left) {
     l2_prefetch(c.URs + (size_t)st * NN, NN);
@@ -161,7 +161,7 @@ __device__ __noinline__ void prefetch_wrap(const ChainDesc &c, int st, bool left
 }
 
 // Local_sweep_L (src/local_sweep.f90:106-124)
-__device__ __noinline__ void sweep_L(const ChainDesc &c, const Smem &s) {
+static __device__ __noinline__ void sweep_L(const ChainDesc &c, const Smem &s) {
   const int N = c.N;
   Pend pd{1, 0};
   for (int nt = c.Ltrot; nt >= 1; --nt) {
@@ -180,7 +180,7 @@ __device__ __noinline__ void sweep_L(const ChainDesc &c, const Smem &s) {
 }
 
 // Local_sweep_R (src/local_sweep.f90:126-150)
-__device__ __noinline__ void sweep_R(const ChainDesc &c, const Smem &s, bool toggle) {
+static __device__ __noinline__ void sweep_R(const ChainDesc &c, const Smem &s, bool toggle) {
   const int N = c.N;
   if (toggle) {
     { PhTimer t(c, PH_DYN); dyn_sweep(c, s); }
@@ -204,12 +204,12 @@ __device__ __noinline__ void sweep_R(const ChainDesc &c, const Smem &s, bool tog
   }
 }
 
-__device__ __noinline__ void bin_average(const ChainDesc &c, bool toggle);
+static __device__ __noinline__ void bin_average(const ChainDesc &c, bool toggle);
 
 // Local_sweep_reset (src/local_sweep.f90:56-71): the bin's sums and
 // acceptance counters, the tau correlators when toggle, and for h = 0 the
 // links made constant in tau.
-__device__ __noinline__ void sweep_reset(const ChainDesc &c, bool toggle, bool h_is_zero) {
+static __device__ __noinline__ void sweep_reset(const ChainDesc &c, bool toggle, bool h_is_zero) {
   const int N = c.N;
   if (threadIdx.x == 0) {
     for (int q = A_FLUX_SUM; q <= A_ACC_DEN; ++q) c.acc[q] = 0.0;
@@ -228,7 +228,7 @@ __device__ __noinline__ void sweep_reset(const ChainDesc &c, bool toggle, bool h
 }
 
 // Local_sweep (src/local_sweep.f90:152-195): one bin.
-__device__ __noinline__ void chain_sweep(const ChainDesc &c, const Smem &s, int nsweep, bool toggle,
+static __device__ __noinline__ void chain_sweep(const ChainDesc &c, const Smem &s, int nsweep, bool toggle,
                             double h_is_zero) {
   sweep_reset(c, toggle, h_is_zero != 0.0);
   load_G(c, s);
@@ -246,7 +246,7 @@ __device__ __noinline__ void chain_sweep(const ChainDesc &c, const Smem &s, int 
 
 // Obs_equal_ave (src/obser_equal.f90:50-71): the bin averages of nobs
 // slices into the chain's readback slots.
-__device__ __noinline__ void obs_equal_ave(const ChainDesc &c, double nobs) {
+static __device__ __noinline__ void obs_equal_ave(const ChainDesc &c, double nobs) {
   const int N = c.N;
   if (threadIdx.x == 0) {
     double *o = c.acc + A_BIN0;
@@ -267,7 +267,7 @@ __device__ __noinline__ void obs_equal_ave(const ChainDesc &c, double nobs) {
 }
 
 // Obs_tau_ave (src/obser_tau.f90:37-47): the tau correlators / nobst.
-__device__ __noinline__ void obs_tau_ave(const ChainDesc &c, double nobst) {
+static __device__ __noinline__ void obs_tau_ave(const ChainDesc &c, double nobst) {
   const double z = 1.0 / nobst;
   const size_t n = (size_t)7 * c.Ltrot * c.N;
   for (size_t i = threadIdx.x; i < n; i += Z2_NT) c.obs_tau[i] = z * c.obs_tau[i];
@@ -276,7 +276,7 @@ __device__ __noinline__ void obs_tau_ave(const ChainDesc &c, double nobst) {
 
 // End of a bin: Obs_equal_ave, Acc_calc_ratio (src/process_matrix.f90:134-140)
 // and, with toggle, Obs_tau_ave, with the counts the half-sweeps kept.
-__device__ __noinline__ void bin_average(const ChainDesc &c, bool toggle) {
+static __device__ __noinline__ void bin_average(const ChainDesc &c, bool toggle) {
   obs_equal_ave(c, c.acc[A_NOBS]);
   if (threadIdx.x == 0 && c.acc[A_ACC_DEN] > 0.0)
     c.acc[A_ACC] += c.acc[A_ACC_NUM] / c.acc[A_ACC_DEN];
@@ -291,7 +291,7 @@ __device__ __noinline__ void bin_average(const ChainDesc &c, bool toggle) {
 // configuration staged in shared memory when it fits (the arena is free
 // before z2_pre).  Acc_Kt%acc accumulates in A_TACC.
 // ---------------------------------------------------------------------------
-__device__ __noinline__ void chain_therm(const ChainDesc &c, const Smem &s, int nwarm) {
+static __device__ __noinline__ void chain_therm(const ChainDesc &c, const Smem &s, int nwarm) {
   const int L = c.Ltrot, nb = c.nb;
   const size_t bytes = (size_t)L * nb;
   const size_t arena = 8 * ((c.g_in_smem ? (size_t)c.N * s.ldg : 0) + (size_t)s.tile_doubles);
@@ -356,7 +356,7 @@ __device__ __forceinline__ int dev_nranf(unsigned int &st, int N) {
 // State of the chain that a rejected move restores (Prop_assign and
 // Wrlist_assign, src/process_matrix.f90:58-66, 104-112): G, UR, VR, ULT, VL
 // (contiguous), DR, DL, the four UDV stacks, their D stacks and Xmaxm.
-__device__ __noinline__ void global_backup(const ChainDesc &c, bool save) {
+static __device__ __noinline__ void global_backup(const ChainDesc &c, bool save) {
   const size_t NN = (size_t)c.N * c.N, S1 = (size_t)c.Nst + 1;
   const size_t n0 = 5 * NN, n1 = 2 * (size_t)c.N, n2 = 4 * NN * S1, n3 = 2 * (size_t)c.N * S1;
   double *src[4] = {c.G, c.DR, c.URs, c.DRs};
@@ -377,7 +377,7 @@ __device__ __noinline__ void global_backup(const ChainDesc &c, bool save) {
 // One cluster site of a trial half-sweep (ratioK_fermion, src/globalK.f90:15-113):
 // the bond flips at slice nt if the cluster holds nt; |det Prod|^2 goes into
 // the fermion log ratio (thread 0) and G takes the rank-2 update.
-__device__ __noinline__ void global_flip_slice(const ChainDesc &c, const Smem &s, int nt, int b,
+static __device__ __noinline__ void global_flip_slice(const ChainDesc &c, const Smem &s, int nt, int b,
                                                double &lrf) {
   if (!c.gmask[nt - 1]) return;
   const int N = c.N, ldg = s.ldg, ldx = s.ldx;
@@ -420,7 +420,7 @@ __device__ __noinline__ void global_flip_slice(const ChainDesc &c, const Smem &s
 // Global_sweep_L's trial (src/global_update.f90:228-272 with GlobalK_prop_L,
 // src/globalK.f90:115-133): the Local_sweep_L structure without observables
 // or drift statistics, the cluster's flips forced.
-__device__ __noinline__ void sweep_L_trial(const ChainDesc &c, const Smem &s, int b, double &lrf) {
+static __device__ __noinline__ void sweep_L_trial(const ChainDesc &c, const Smem &s, int b, double &lrf) {
   const int N = c.N;
   Pend pd{1, 0};
   for (int nt = c.Ltrot; nt >= 1; --nt) {
@@ -438,7 +438,7 @@ __device__ __noinline__ void sweep_L_trial(const ChainDesc &c, const Smem &s, in
 
 // Global_sweep_R's trial (src/global_update.f90:274-318, GlobalK_prop_R,
 // src/globalK.f90:135-153).
-__device__ __noinline__ void sweep_R_trial(const ChainDesc &c, const Smem &s, int b, double &lrf) {
+static __device__ __noinline__ void sweep_R_trial(const ChainDesc &c, const Smem &s, int b, double &lrf) {
   const int N = c.N;
   Pend pd{1, 0};
   { PhTimer t(c, PH_WRAP); wrap_R(c, s, 0, pd, false); }
@@ -455,7 +455,7 @@ __device__ __noinline__ void sweep_R_trial(const ChainDesc &c, const Smem &s, in
 }
 
 // Global_sweep (src/global_update.f90:320-337): nglobal Wolff moves.
-__device__ __noinline__ void chain_global(const ChainDesc &c, const Smem &s, int nglobal) {
+static __device__ __noinline__ void chain_global(const ChainDesc &c, const Smem &s, int nglobal) {
   const int L = c.Ltrot, nb = c.nb;
   double *gs = s.red + 40;   // [0] bond, [1] size, [2] log ratio space, [3] accept
   int num = 0;
@@ -578,7 +578,7 @@ __device__ __forceinline__ double grad_block(double x11, double x12, double x21,
 //   (through E2, the second also through E3);  state 2: second E2 (through
 //   E2^-1), second E1;  state 3: second E0 (through E0^-1).
 // A group has one term per bond, so its bonds are spread over the threads.
-__device__ __noinline__ void grad_groups(const ChainDesc &c, const Smem &s, int nt, int state) {
+static __device__ __noinline__ void grad_groups(const ChainDesc &c, const Smem &s, int nt, int state) {
   const int ldg = s.ldg, half = c.half;
   const double *G = s.G;
   const double hd = -0.5 * c.dtau;
@@ -637,7 +637,7 @@ __device__ __noinline__ void grad_groups(const ChainDesc &c, const Smem &s, int 
   __syncthreads();
 }
 
-__device__ __noinline__ void chain_logdet_grad(const ChainDesc &c, const Smem &s) {
+static __device__ __noinline__ void chain_logdet_grad(const ChainDesc &c, const Smem &s) {
   const int N = c.N;
   for (int b = threadIdx.x; b < c.nb; b += Z2_NT) c.grad[b] = 0.0;
   __syncthreads();

@@ -19,7 +19,7 @@ __device__ __forceinline__ size_t xy_at(int i, int q, int ldx) {
 // chunks of 4 columns, reusing each X fragment TC times and each Yt fragment
 // TR times.
 template <bool GS, int TR, int TC>
-__device__ __noinline__ void flush_tiles(double *G, int ldg, const double *X, const double *Yt,
+static __device__ __noinline__ void flush_tiles(double *G, int ldg, const double *X, const double *Yt,
                                          int N, int ldx, int m) {
   if (GS) G = as_shared(G);
   X = as_shared(X);
@@ -79,7 +79,7 @@ __device__ __noinline__ void flush_tiles(double *G, int ldg, const double *X, co
 
 // The same update for any N: (8 GS) x (8 GS) groups with bounds checks.
 template <bool SH, int GS>
-__device__ __noinline__ void flush_generic(double *G, int ldg, const double *X, const double *Yt,
+static __device__ __noinline__ void flush_generic(double *G, int ldg, const double *X, const double *Yt,
                                            int N, int ldx, int m) {
   if (SH) G = as_shared(G);
   X = as_shared(X);

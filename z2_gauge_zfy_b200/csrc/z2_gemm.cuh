@@ -112,7 +112,7 @@ __device__ __forceinline__ void gemm_unit(int n, MatRef A, MatRef B, int r0, int
 
 // C = A B (out), n % 4 == 0; rowmap (optional): row i of A is its row rowmap[i].
 template <int RT, int CT, bool VA, bool VB, int TRI>
-__device__ __noinline__ void gemm_units(int n, MatRef A, const int *rowmap, MatRef B, const GemmOut &out) {
+static __device__ __noinline__ void gemm_units(int n, MatRef A, const int *rowmap, MatRef B, const GemmOut &out) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int lr = lane >> 2, lc = lane & 3;
   const int tiles = (n + 7) >> 3;
@@ -175,7 +175,7 @@ __device__ __forceinline__ void gemm_sized(int n, MatRef A, const int *rowmap, M
 // allow: N = 144 takes 80 K cycles against 103 K for 16 x 16 groups (47 K at the
 // SM's DMMA rate; the fragment loads' trips to L2 are the rest).  a_upper: A(i, l) reads as 0 for i > l; b_lower: B(l, j) reads as 0 for
 // l < j.
-__device__ __noinline__ void gemm_nnn(int n, MatRef A, const int *rowmap, bool a_upper, MatRef B,
+static __device__ __noinline__ void gemm_nnn(int n, MatRef A, const int *rowmap, bool a_upper, MatRef B,
                                       bool b_lower, GemmOut out) {
   const bool va = A.cs == 1 && (A.rs & 1) == 0 && ((uintptr_t)A.p & 15) == 0;
   const bool vb = B.rs == 1 && (B.cs & 1) == 0 && ((uintptr_t)B.p & 15) == 0;

@@ -42,7 +42,7 @@ __device__ __forceinline__ void load_desc(ChainDesc &sc, const ChainDesc *g) {
 
 #if Z2_NT == 256
 // A module procedure on single matrices, one CTA.
-__device__ __noinline__ void unit_op(const ChainDesc &sc, const Smem &s, int op, const UnitArgs &a) {
+static __device__ __noinline__ void unit_op(const ChainDesc &sc, const Smem &s, int op, const UnitArgs &a) {
   const int N = sc.N;
   if (op == U_MMULT_R || op == U_MMULT_L) {
     build_table(sc, s, a.nt);
@@ -64,7 +64,7 @@ __device__ __noinline__ void unit_op(const ChainDesc &sc, const Smem &s, int op,
 }
 
 // A procedure of the reference's modules on a chain's resident state, one CTA.
-__device__ __noinline__ void state_op(const ChainDesc &c, const Smem &s, int op, int nt, int flag, double x) {
+static __device__ __noinline__ void state_op(const ChainDesc &c, const Smem &s, int op, int nt, int flag, double x) {
   const int N = c.N;
   Pend pd{1, 0};
   switch (op) {

@@ -29,7 +29,7 @@ __device__ __forceinline__ int kin_pass_group(int p) { return p < 4 ? p : 7 - p;
 // The part of the slice table that does not change: position q = g half + k
 // holds bond groups[q]: its sites, C, sinh (in S's place) and, in gid, the bond
 // with the sign of sinh on top.  Once per launch and chain.
-__device__ __noinline__ void kin_init(const ChainDesc &c, const Smem &s) {
+static __device__ __noinline__ void kin_init(const ChainDesc &c, const Smem &s) {
   for (int q = threadIdx.x; q < c.nb; q += Z2_NT) {
     const int b = c.groups[q];
     const double sh = c.chsh[2 * b + 1];
@@ -54,7 +54,7 @@ __device__ __forceinline__ void build_table_on(const signed char *sg, int nb, do
   __syncthreads();
 }
 
-__device__ __noinline__ void build_table(const ChainDesc &c, const Smem &s, int nt) {
+static __device__ __noinline__ void build_table(const ChainDesc &c, const Smem &s, int nt) {
   build_table_on(c.sigma + (size_t)(nt - 1) * c.nb, c.nb, as_shared(s.cs), as_shared(s.gid));
 }
 
@@ -158,7 +158,7 @@ __device__ __forceinline__ void kin_sweep_on(const double2 *cs, double *M, int l
 }
 
 template <bool ROWS, bool Y, int L>
-__device__ __noinline__ void kin_sweep(const double2 *cs, double *M, int ld, int n, int Lx, int Ly, double fl,
+static __device__ __noinline__ void kin_sweep(const double2 *cs, double *M, int ld, int n, int Lx, int Ly, double fl,
                                        bool before, bool after) {
   kin_sweep_on<ROWS, Y, L>(as_shared(const_cast<double2 *>(cs)), as_shared(M), ld, n, Lx, Ly, fl, before, after);
 }
@@ -234,7 +234,7 @@ __device__ __forceinline__ void kin_groups(const ChainDesc &c, const Smem &s, do
 // is called then) passes through shared memory in slabs of columns or rows, one
 // read and one write instead of one of each per sweep.
 template <bool ROWS>
-__device__ __noinline__ void kin_apply(const ChainDesc &c, const Smem &s, double *M, int ld, int n, int nflag,
+static __device__ __noinline__ void kin_apply(const ChainDesc &c, const Smem &s, double *M, int ld, int n, int nflag,
                                        int k0, int k1) {
   const double fl = (double)nflag;
   const int N = c.N;
@@ -273,7 +273,7 @@ __device__ __forceinline__ void kin_cols(const ChainDesc &c, const Smem &s, doub
 // the whole of it: a call costs its registers' round trip through local
 // memory, which on small lattices was as much as a sweep.
 template <int L>
-__device__ __noinline__ void kin_square(const ChainDesc &c, const Smem &s, double *M, int ld, int t0, int t1,
+static __device__ __noinline__ void kin_square(const ChainDesc &c, const Smem &s, double *M, int ld, int t0, int t1,
                                         int dt, int rf, int cf) {
   M = as_shared(M);
   double2 *cs = as_shared(s.cs);
@@ -324,7 +324,7 @@ __device__ __forceinline__ void kin_slices(const ChainDesc &c, const Smem &s, do
 
 // Apply B-multiplications to a global N x N matrix, staging it through the
 // arena when it fits (the arena must be free).
-__device__ __noinline__ void kin_global(const ChainDesc &c, const Smem &s, double *M, int row_flag,
+static __device__ __noinline__ void kin_global(const ChainDesc &c, const Smem &s, double *M, int row_flag,
                                         int col_flag) {
   const int N = c.N;
   if (c.g_in_smem) {

@@ -52,7 +52,7 @@ __device__ __forceinline__ void blk_walk(int m, int n, Ld ld, Use use) {
 // (m, both leading dimensions even and both pointers 16-byte aligned), dealt
 // out flat over the block: the copies wait on L2, 144 x 144 took 20 K cycles as
 // one column per warp with four loads in flight.
-__device__ __noinline__ void blk_copy(double *dst, int ldd, const double *src, int lds, int m, int n) {
+static __device__ __noinline__ void blk_copy(double *dst, int ldd, const double *src, int lds, int m, int n) {
   if (!((m | ldd | lds) & 1) && !(((size_t)dst | (size_t)src) & 15)) {
     double2 *d = reinterpret_cast<double2 *>(dst);
     const double2 *s = reinterpret_cast<const double2 *>(src);
@@ -69,27 +69,27 @@ __device__ __noinline__ void blk_copy(double *dst, int ldd, const double *src, i
   __syncthreads();
 }
 // dst = src^T (src m x n -> dst n x m)
-__device__ __noinline__ void blk_transpose(double *dst, int ldd, const double *src, int lds, int m, int n) {
+static __device__ __noinline__ void blk_transpose(double *dst, int ldd, const double *src, int lds, int m, int n) {
   for (int j = threadIdx.x / 32; j < m; j += Z2_WARPS)
     for (int i = threadIdx.x & 31; i < n; i += 32) dst[i + (size_t)j * ldd] = src[j + (size_t)i * lds];
   __syncthreads();
 }
-__device__ __noinline__ void blk_identity(double *A, int lda, int n) {
+static __device__ __noinline__ void blk_identity(double *A, int lda, int n) {
   for (int j = threadIdx.x / 32; j < n; j += Z2_WARPS)
     for (int i = threadIdx.x & 31; i < n; i += 32) A[i + (size_t)j * lda] = (i == j) ? 1.0 : 0.0;
   __syncthreads();
 }
-__device__ __noinline__ void blk_fill(double *v, int n, double x) {
+static __device__ __noinline__ void blk_fill(double *v, int n, double x) {
   for (int i = threadIdx.x; i < n; i += Z2_NT) v[i] = x;
   __syncthreads();
 }
-__device__ __noinline__ void blk_scale(double *A, int lda, int m, int n, double a) {
+static __device__ __noinline__ void blk_scale(double *A, int lda, int m, int n, double a) {
   for (int j = threadIdx.x / 32; j < n; j += Z2_WARPS)
     for (int i = threadIdx.x & 31; i < m; i += 32) A[i + (size_t)j * lda] *= a;
   __syncthreads();
 }
 // A(:, j) *= d(j)
-__device__ __noinline__ void blk_scale_cols(double *A, int lda, int m, int n, const double *d) {
+static __device__ __noinline__ void blk_scale_cols(double *A, int lda, int m, int n, const double *d) {
   for (int j = threadIdx.x / 32; j < n; j += Z2_WARPS) {
     double dj = d[j];
     for (int i = threadIdx.x & 31; i < m; i += 32) A[i + (size_t)j * lda] *= dj;
@@ -102,7 +102,7 @@ __device__ __noinline__ void blk_scale_cols(double *A, int lda, int m, int n, co
 // On exit A holds R and the reflectors, tau the scalar factors, jpvt the
 // 1-based pivots (column j of A*P is column jpvt(j) of A).
 // ---------------------------------------------------------------------------
-__device__ __noinline__ void blk_geqp3(double *A, int lda, int n, int *jpvt, double *tau, double *vn1,
+static __device__ __noinline__ void blk_geqp3(double *A, int lda, int n, int *jpvt, double *tau, double *vn1,
                           double *vn2) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const double tol3z = 1.0536712127723509e-08;   // sqrt(dlamch('E')) = sqrt(2^-53)
@@ -195,7 +195,7 @@ __device__ __noinline__ void blk_geqp3(double *A, int lda, int n, int *jpvt, dou
 // R(i, i:n) /= D(i).
 // The rows are scaled by the reciprocal of D (one division per row instead
 // of one per element; rd: n doubles of scratch, left holding 1/D).
-__device__ __noinline__ void blk_qdrp_scale(double *A, int lda, int n, double *D, double *rd) {
+static __device__ __noinline__ void blk_qdrp_scale(double *A, int lda, int n, double *D, double *rd) {
   for (int i = threadIdx.x; i < n; i += Z2_NT) {
     const double d = fabs(A[i + (size_t)i * lda]);
     D[i] = d;
@@ -209,7 +209,7 @@ __device__ __noinline__ void blk_qdrp_scale(double *A, int lda, int n, double *D
 
 // Row / column permutations with 1-based pivots (ZLAPMR, ZLAPMT).
 // forward row: dst(i,:) = src(jpvt(i),:) ; backward row: dst(jpvt(i),:) = src(i,:)
-__device__ __noinline__ void blk_perm_rows(double *dst, int ldd, const double *src, int lds, int n, int nc,
+static __device__ __noinline__ void blk_perm_rows(double *dst, int ldd, const double *src, int lds, int n, int nc,
                               const int *jpvt, bool forward) {
   for (int j = threadIdx.x / 32; j < nc; j += Z2_WARPS)
     for (int i = threadIdx.x & 31; i < n; i += 32) {
@@ -220,7 +220,7 @@ __device__ __noinline__ void blk_perm_rows(double *dst, int ldd, const double *s
   __syncthreads();
 }
 // forward col: dst(:,j) = src(:,jpvt(j)) ; backward col: dst(:,jpvt(j)) = src(:,j)
-__device__ __noinline__ void blk_perm_cols(double *dst, int ldd, const double *src, int lds, int nr, int n,
+static __device__ __noinline__ void blk_perm_cols(double *dst, int ldd, const double *src, int lds, int nr, int n,
                               const int *jpvt, bool forward) {
   for (int j = threadIdx.x / 32; j < n; j += Z2_WARPS) {
     int p = jpvt[j] - 1;

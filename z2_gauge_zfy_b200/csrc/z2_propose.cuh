@@ -44,7 +44,7 @@ __device__ __forceinline__ unsigned int ranf_pow(int n) {
 // picking the accepted rows and columns out of the registers.
 // GS: G is in shared memory.
 template <bool GS>
-__device__ __noinline__ void propose_window(const ChainDesc &c, const Smem &s, int nt,
+static __device__ __noinline__ void propose_window(const ChainDesc &c, const Smem &s, int nt,
                                             bool descending, int dir) {
   const int N = c.N, nb = c.nb, k2 = c.k2, Lt = c.Ltrot;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;

@@ -163,7 +163,7 @@ __device__ __forceinline__ void qrp_colsum8(double (&d)[S], int tr, int hl) {
 
 // work: >= 2 n doubles (reflector + two int maps); red: >= 32 doubles.
 template <int S>
-__device__ __noinline__ void qrp_reg(double *A, int lda, int n, int *jpvt, double *tau,
+static __device__ __noinline__ void qrp_reg(double *A, int lda, int n, int *jpvt, double *tau,
                                      double *vn1, double *vn2, double *work, double *red) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int tr = lane & 15, tc = (warp << 1) | (lane >> 4);

@@ -14,7 +14,7 @@ __device__ __forceinline__ void mul_nn(int n, MatRef A, bool a_upper, MatRef B, 
 
 // The orthogonal factor of reflectors with coefficients tau (the pivoted QR),
 // in place; vd: n doubles of shared memory.
-__device__ __noinline__ void form_q(double *A, int lda, int n, const double *tau, double *vd,
+static __device__ __noinline__ void form_q(double *A, int lda, int n, const double *tau, double *vd,
                                     double *work, int wd) {
   if (wd < wy_work(n)) {
     blk_org2r_tc(A, lda, n, n, tau);
@@ -31,7 +31,7 @@ __device__ __noinline__ void form_q(double *A, int lda, int n, const double *tau
 // On entry A (lda; shared arena or global) holds the propagated U (UR, or
 // UL^T).  U, D, V are the factors in global memory (U = UR or UL^T); W0 is an
 // N x N global workspace.
-__device__ __noinline__ void dev_stab_U(const Smem &s, int N, double *A, int lda, double *U,
+static __device__ __noinline__ void dev_stab_U(const Smem &s, int N, double *A, int lda, double *U,
                                         double *D, double *V, double *W0, bool left) {
   double *tau = s.vec, *vn1 = s.vec + N, *vn2 = s.vec + 2 * N, *Dn = s.vec + 3 * N;
   int *jpvt = s.ivec;
@@ -58,7 +58,7 @@ __device__ __noinline__ void dev_stab_U(const Smem &s, int N, double *A, int lda
 // (DMMA-blocked) and the permutation follow in the reference's order.
 // M (ldm) is the QR work matrix (shared arena when it fits); W1, W2, W3 are
 // N x N global workspaces (W3 keeps the scaled R).
-__device__ __noinline__ void dev_stab_green(const Smem &s, int N, int nt, int Ltrot,
+static __device__ __noinline__ void dev_stab_green(const Smem &s, int N, int nt, int Ltrot,
                                             const double *UR, const double *DR,
                                             const double *VR, const double *ULT,
                                             const double *DL, const double *VL, double *M,
@@ -175,7 +175,7 @@ __device__ __forceinline__ void gj_any(double *M, int ldm, int n, int *piv, doub
 // A <- A P S, column j of it being sc[j] (null: 1) times column perm[j] of A, in
 // shared memory through registers (n <= 32 T).
 template <int T>
-__device__ __noinline__ void permute_cols_reg(double *A, int lda, int n, const int *perm, const double *sc) {
+static __device__ __noinline__ void permute_cols_reg(double *A, int lda, int n, const int *perm, const double *sc) {
   A = as_shared(A);
   constexpr int C = 32 * T / Z2_WARPS;    // columns per warp
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -258,7 +258,7 @@ __device__ __forceinline__ void scale_upper(double *A, int lda, int n, const dou
 // stab_UR / stab_UL with the pre-pivoted QR; arguments as dev_stab_U.  D scales
 // the columns of A, which leaves Q as it is and scales R's columns, so A itself
 // is factored and D meets only the column order and R.
-__device__ __noinline__ void dev_stab_U_fast(const Smem &s, int N, double *A, int lda, double *U,
+static __device__ __noinline__ void dev_stab_U_fast(const Smem &s, int N, double *A, int lda, double *U,
                                              double *D, double *V, double *W0, bool left) {
   if (!wy_ok(N, s.tile_doubles)) {
     dev_stab_U(s, N, A, lda, U, D, V, W0, left);
@@ -319,7 +319,7 @@ __device__ __noinline__ void dev_stab_U_fast(const Smem &s, int N, double *A, in
 // receive DRb^-1, DLb^-1, DRs, DLs (N doubles of shared memory each).  N a
 // multiple of 4; above the panel kernels' range the inverse comes from a
 // blocked LU through the N x N global workspaces W0, W1.
-__device__ __noinline__ void middle_inverse(const Smem &s, int N, const double *UR, const double *DR,
+static __device__ __noinline__ void middle_inverse(const Smem &s, int N, const double *UR, const double *DR,
                                             const double *VR, const double *ULT, const double *DL,
                                             const double *VL, double *M, int ldm, double *rRb,
                                             double *rLb, double *Rs, double *Ls, int *piv, double *W0,
@@ -345,7 +345,7 @@ __device__ __noinline__ void middle_inverse(const Smem &s, int N, const double *
 
 // stab_green with the scale-split middle matrix; arguments as dev_stab_green
 // (W1 and W2 are N x N scratch).
-__device__ __noinline__ void dev_stab_green_fast(const Smem &s, int N, int nt, int Ltrot,
+static __device__ __noinline__ void dev_stab_green_fast(const Smem &s, int N, int nt, int Ltrot,
                                                  const double *UR, const double *DR,
                                                  const double *VR, const double *ULT,
                                                  const double *DL, const double *VL, double *M,
