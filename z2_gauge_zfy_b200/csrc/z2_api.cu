@@ -1279,6 +1279,8 @@ extern "C" int z2_stab_green_big(z2_handle *h, int32_t chain, const double *UR, 
 // the same order).  One CTA, the chain kernel's shared-memory plan.
 // ---------------------------------------------------------------------------
 
+// Launch one state procedure on one chain, synchronously; a non-finite drift
+// or Green's function found by it is Z2_ERR_NONFINITE.
 static int run_state(z2_handle *h, int chain, int op, int nt, int flag, double x) {
   CUDA_TRY(h, cudaSetDevice(h->device));
   ModArgs m{};

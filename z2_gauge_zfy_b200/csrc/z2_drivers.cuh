@@ -73,10 +73,9 @@ static __device__ __noinline__ void dyn_reset(const ChainDesc &c, const Smem &s)
 static __device__ __noinline__ void propgr_R(const ChainDesc &c, const Smem &s, int nt, bool kin, bool mu) {
   const int N = c.N;
   if (kin && c.use_kin) {
-    build_table(c, s, nt);
-    kin_global(c, s, c.Gt0, 1, 0);
-    kin_global(c, s, c.G0t, 0, -1);
-    kin_global(c, s, c.Gtt, 1, -1);
+    kin_global(c, s, nt, c.Gt0, 1, 0);
+    kin_global(c, s, nt, c.G0t, 0, -1);
+    kin_global(c, s, nt, c.Gtt, 1, -1);
   }
   if (mu && (c.eP != 1.0 || c.eM != 1.0)) {
     blk_scale(c.Gt0, N, N, N, c.eP);

@@ -45,9 +45,9 @@ __device__ __forceinline__ void load_desc(ChainDesc &sc, const ChainDesc *g) {
 static __device__ __noinline__ void unit_op(const ChainDesc &sc, const Smem &s, int op, const UnitArgs &a) {
   const int N = sc.N;
   if (op == U_MMULT_R || op == U_MMULT_L) {
-    build_table(sc, s, a.nt);
-    if (op == U_MMULT_R) kin_global(sc, s, a.M, a.nflag, 0);
-    else kin_global(sc, s, a.M, 0, a.nflag);
+    kin_init(sc, s);
+    if (op == U_MMULT_R) kin_global(sc, s, a.nt, a.M, a.nflag, 0);
+    else kin_global(sc, s, a.nt, a.M, 0, a.nflag);
   } else if (op == U_STAB_UR || op == U_STAB_UL) {
     int lda; double *A = qr_matrix(sc, s, lda);
     blk_copy(A, lda, a.U, N, N, N);
@@ -67,28 +67,31 @@ static __device__ __noinline__ void unit_op(const ChainDesc &sc, const Smem &s, 
 static __device__ __noinline__ void state_op(const ChainDesc &c, const Smem &s, int op, int nt, int flag, double x) {
   const int N = c.N;
   Pend pd{1, 0};
+  switch (op) {      // the slice table is set up for the procedures that use it
+    case SO_PROPK_PRE: case SO_PROPK_L: case SO_PROPK_R: case SO_PROPGRK_R: case SO_SLICE_L: case SO_SLICE_R:
+      kin_init(c, s);
+      break;
+    default:
+      break;
+  }
   switch (op) {
     case SO_PROPK_PRE:      // propK_pre (src/multiply.f90:8-15) as Local_sweep_pre calls it
-      if (c.use_kin) { build_table(c, s, nt); kin_global(c, s, c.UR, 1, 0); }
+      if (c.use_kin) kin_global(c, s, nt, c.UR, 1, 0);
       break;
     case SO_PROPT_PRE:      // propT_pre (src/multiply.f90:65-77)
       blk_scale(c.UR, N, N, N, c.eP);
       break;
     case SO_PROPK_L:        // propK_L (src/multiply.f90:17-28): G B, B^-1 G, UL B
       load_G(c, s);
-      build_table(c, s, nt);
-      kin_cols(c, s, s.G, s.ldg, N, 1);
-      kin_rows(c, s, s.G, s.ldg, N, -1);
+      kin_slices(c, s, s.G, s.ldg, nt, nt, 1, -1, 1);   // B^-1 G B
       spill_G(c, s);
-      kin_global(c, s, c.ULT, 1, 0);      // UL^T <- B UL^T (B symmetric)
+      kin_global(c, s, nt, c.ULT, 1, 0);      // UL^T <- B UL^T (B symmetric)
       break;
     case SO_PROPK_R:        // propK_R (src/multiply.f90:30-41): B G, G B^-1, B UR
       load_G(c, s);
-      build_table(c, s, nt);
-      kin_rows(c, s, s.G, s.ldg, N, 1);
-      kin_cols(c, s, s.G, s.ldg, N, -1);
+      kin_slices(c, s, s.G, s.ldg, nt, nt, 1, 1, -1);   // B G B^-1
       spill_G(c, s);
-      kin_global(c, s, c.UR, 1, 0);
+      kin_global(c, s, nt, c.UR, 1, 0);
       break;
     case SO_PROPT_L:        // propT_L (src/multiply.f90:79-93)
       blk_scale(c.G, N, N, N, c.eP);
@@ -103,7 +106,7 @@ static __device__ __noinline__ void state_op(const ChainDesc &c, const Smem &s, 
     case SO_PROPGRK_R:      // propgrK_R (src/multiply.f90:43-63) on the Dyn copy
       if (c.use_kin) {
         propgr_R(c, s, nt, true, false);
-        kin_global(c, s, c.URd, 1, 0);
+        kin_global(c, s, nt, c.URd, 1, 0);
       }
       break;
     case SO_PROPGRT_R:      // propgrT_R (src/multiply.f90:110-130)
@@ -150,28 +153,20 @@ static __device__ __noinline__ void state_op(const ChainDesc &c, const Smem &s, 
       load_G(c, s);
       if (op == SO_SLICE_L) {
         propose_slice(c, s, nt, true, 0);            // bonds 2N..1
-        build_table(c, s, nt);
-        kin_cols(c, s, s.G, s.ldg, N, 1);
-        kin_rows(c, s, s.G, s.ldg, N, -1);
+        kin_slices(c, s, s.G, s.ldg, nt, nt, 1, -1, 1);   // B^-1 G B
         spill_G(c, s);
-        kin_global(c, s, c.ULT, 1, 0);
+        kin_global(c, s, nt, c.ULT, 1, 0);
       } else {
-        build_table(c, s, nt);
-        kin_rows(c, s, s.G, s.ldg, N, 1);
-        kin_cols(c, s, s.G, s.ldg, N, -1);
+        kin_slices(c, s, s.G, s.ldg, nt, nt, 1, 1, -1);   // B G B^-1
         propose_slice(c, s, nt, false, 1);           // bonds 1..2N
         spill_G(c, s);
-        build_table(c, s, nt);                       // B_nt with the flipped links
-        kin_global(c, s, c.UR, 1, 0);
+        kin_global(c, s, nt, c.UR, 1, 0);            // B_nt with the flipped links
       }
       break;
     default:
       break;
   }
 }
-
-// Launch one state procedure on one chain, synchronously; a non-finite drift
-// or Green's function found by it is Z2_ERR_NONFINITE.
 
 #endif
 
@@ -197,7 +192,7 @@ z2_chain_kernel(const ChainDesc *descs, const int *order, int nchains, int *queu
     }
     if (threadIdx.x == 0) s = make_smem(sc, z2_smem, smem_bytes);
     __syncthreads();
-    if (op != OP_THERM) kin_init(sc, s);
+    if (op != OP_THERM && op != OP_UNIT && op != OP_STATE) kin_init(sc, s);
     if (op == OP_PRE) {
       chain_pre(sc, s);
     } else if (op == OP_SWEEP) {

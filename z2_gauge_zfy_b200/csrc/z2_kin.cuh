@@ -322,19 +322,17 @@ __device__ __forceinline__ void kin_slices(const ChainDesc &c, const Smem &s, do
   }
 }
 
-// Apply B-multiplications to a global N x N matrix, staging it through the
-// arena when it fits (the arena must be free).
-static __device__ __noinline__ void kin_global(const ChainDesc &c, const Smem &s, double *M, int row_flag,
-                                        int col_flag) {
+// M <- B_nt^row_flag M, then M <- M B_nt^col_flag (0: not) of a global N x N matrix,
+// staged through the arena when it fits (the arena must be free).
+static __device__ __noinline__ void kin_global(const ChainDesc &c, const Smem &s, int nt, double *M,
+                                               int row_flag, int col_flag) {
   const int N = c.N;
   if (c.g_in_smem) {
     double *A = s.arena;
     blk_copy(A, c.ldg, M, N, N, N);
-    if (row_flag) kin_rows(c, s, A, c.ldg, N, row_flag);
-    if (col_flag) kin_cols(c, s, A, c.ldg, N, col_flag);
+    kin_slices(c, s, A, c.ldg, nt, nt, 1, row_flag, col_flag);
     blk_copy(M, N, A, c.ldg, N, N);
   } else {
-    if (row_flag) kin_rows(c, s, M, N, N, row_flag);
-    if (col_flag) kin_cols(c, s, M, N, N, col_flag);
+    kin_slices(c, s, M, N, nt, nt, 1, row_flag, col_flag);
   }
 }
