@@ -157,23 +157,24 @@ __device__ __forceinline__ void kin_sweep_on(const double2 *cs, double *M, int l
   __syncthreads();
 }
 
-template <bool ROWS, bool Y, int L>
+template <bool ROWS, bool Y, int L, bool SH>
 static __device__ __noinline__ void kin_sweep(const double2 *cs, double *M, int ld, int n, int Lx, int Ly, double fl,
                                        bool before, bool after) {
-  kin_sweep_on<ROWS, Y, L>(as_shared(const_cast<double2 *>(cs)), as_shared(M), ld, n, Lx, Ly, fl, before, after);
+  kin_sweep_on<ROWS, Y, L>(as_shared(const_cast<double2 *>(cs)), SH ? as_shared(M) : M, ld, n, Lx, Ly, fl, before,
+                           after);
 }
 
-template <bool ROWS, bool Y>
+template <bool ROWS, bool Y, bool SH>
 __device__ __forceinline__ void kin_sweep_any(const Smem &s, double *M, int ld, int n, int Lx, int Ly, double fl,
                                               bool before, bool after) {
   switch (Y ? Ly : Lx) {
-    case 4: kin_sweep<ROWS, Y, 4>(s.cs, M, ld, n, Lx, Ly, fl, before, after); return;
-    case 6: kin_sweep<ROWS, Y, 6>(s.cs, M, ld, n, Lx, Ly, fl, before, after); return;
-    case 8: kin_sweep<ROWS, Y, 8>(s.cs, M, ld, n, Lx, Ly, fl, before, after); return;
-    case 10: kin_sweep<ROWS, Y, 10>(s.cs, M, ld, n, Lx, Ly, fl, before, after); return;
-    case 12: kin_sweep<ROWS, Y, 12>(s.cs, M, ld, n, Lx, Ly, fl, before, after); return;
-    case 14: kin_sweep<ROWS, Y, 14>(s.cs, M, ld, n, Lx, Ly, fl, before, after); return;
-    case 16: kin_sweep<ROWS, Y, 16>(s.cs, M, ld, n, Lx, Ly, fl, before, after); return;
+    case 4: kin_sweep<ROWS, Y, 4, SH>(s.cs, M, ld, n, Lx, Ly, fl, before, after); return;
+    case 6: kin_sweep<ROWS, Y, 6, SH>(s.cs, M, ld, n, Lx, Ly, fl, before, after); return;
+    case 8: kin_sweep<ROWS, Y, 8, SH>(s.cs, M, ld, n, Lx, Ly, fl, before, after); return;
+    case 10: kin_sweep<ROWS, Y, 10, SH>(s.cs, M, ld, n, Lx, Ly, fl, before, after); return;
+    case 12: kin_sweep<ROWS, Y, 12, SH>(s.cs, M, ld, n, Lx, Ly, fl, before, after); return;
+    case 14: kin_sweep<ROWS, Y, 14, SH>(s.cs, M, ld, n, Lx, Ly, fl, before, after); return;
+    case 16: kin_sweep<ROWS, Y, 16, SH>(s.cs, M, ld, n, Lx, Ly, fl, before, after); return;
     default: return;
   }
 }
@@ -215,11 +216,11 @@ __device__ __forceinline__ void kin_group_vec(const Smem &s, double *base, size_
 
 // Sweep K (0: groups 0 1; 1: groups 2 3 3 2; 2: groups 1 0) of M <- B^nflag M
 // (rows) or M <- M B^nflag, M in shared memory and fit for the line sweeps.
-template <bool ROWS>
+template <bool ROWS, bool SH>
 __device__ __forceinline__ void kin_lines(const ChainDesc &c, const Smem &s, double *M, int ld, int n, double fl,
                                           int K) {
-  if (K == 1) kin_sweep_any<ROWS, true>(s, M, ld, n, c.Lx, c.Ly, fl, true, true);
-  else kin_sweep_any<ROWS, false>(s, M, ld, n, c.Lx, c.Ly, fl, K == 0, K == 2);
+  if (K == 1) kin_sweep_any<ROWS, true, SH>(s, M, ld, n, c.Lx, c.Ly, fl, true, true);
+  else kin_sweep_any<ROWS, false, SH>(s, M, ld, n, c.Lx, c.Ly, fl, K == 0, K == 2);
 }
 template <bool ROWS>
 __device__ __forceinline__ void kin_groups(const ChainDesc &c, const Smem &s, double *M, int ld, int n, double fl,
@@ -230,31 +231,35 @@ __device__ __forceinline__ void kin_groups(const ChainDesc &c, const Smem &s, do
   __syncthreads();
 }
 // Sweeps k0 <= K < k1 of M <- B^nflag M for n columns (ROWS) or M <- M B^nflag for
-// n rows.  A matrix in global memory (N > 144; the arena is free whenever this
-// is called then) passes through shared memory in slabs of columns or rows, one
-// read and one write instead of one of each per sweep.
+// n rows.  In global memory (N > 144; the arena is free whenever this is called
+// then) B M passes through shared memory in slabs of columns, one read and one
+// write instead of one of each per sweep; M B, whose loads are whole lines of row
+// pairs, sweeps in place (16x16: B M 207 us in place, 96 in slabs; M B 53 and 104).
 template <bool ROWS>
 static __device__ __noinline__ void kin_apply(const ChainDesc &c, const Smem &s, double *M, int ld, int n, int nflag,
                                        int k0, int k1) {
   const double fl = (double)nflag;
   const int N = c.N;
-  const bool lines = c.kin_lines && ((ld | n) & 1) == 0 && ((size_t)M & 15) == 0;
-  if (lines && __isShared(M)) {
-    for (int k = k0; k < k1; ++k) kin_lines<ROWS>(c, s, M, ld, n, fl, k);
-    return;
-  }
-  // slab: w columns at leading dimension N + 2, or w rows at w + 2
-  const int w = (s.tile_doubles / (N + 2) - 2) & ~1;
-  if (lines && !c.g_in_smem && w >= 16) {
-    for (int i = 0; i < n; i += w) {
-      const int m = min(w, n - i);
-      double *src = ROWS ? M + (size_t)i * ld : M + i;
-      const int lt = ROWS ? N + 2 : m + 2;
-      blk_copy(s.tile, lt, src, ld, ROWS ? N : m, ROWS ? m : N);
-      for (int k = k0; k < k1; ++k) kin_lines<ROWS>(c, s, s.tile, lt, m, fl, k);
-      blk_copy(src, ld, s.tile, lt, ROWS ? N : m, ROWS ? m : N);
+  if (c.kin_lines && ((ld | n) & 1) == 0 && ((size_t)M & 15) == 0) {
+    if (__isShared(M)) {
+      for (int k = k0; k < k1; ++k) kin_lines<ROWS, true>(c, s, M, ld, n, fl, k);
+      return;
     }
-    return;
+    if constexpr (Z2_NMAX > 64 && !ROWS) {
+      for (int k = k0; k < k1; ++k) kin_lines<false, false>(c, s, M, ld, n, fl, k);
+      return;
+    }
+    const int w = (s.tile_doubles / (N + 2) - 2) & ~1;      // columns of a slab
+    if (Z2_NMAX > 64 && !c.g_in_smem && w >= 16) {
+      for (int i = 0; i < n; i += w) {
+        const int m = min(w, n - i);
+        double *src = M + (size_t)i * ld;
+        blk_copy(s.tile, N + 2, src, ld, N, m);
+        for (int k = k0; k < k1; ++k) kin_lines<ROWS, true>(c, s, s.tile, N + 2, m, fl, k);
+        blk_copy(src, ld, s.tile, N + 2, N, m);
+      }
+      return;
+    }
   }
   const int p[4] = {0, 2, 6, 8};
   kin_groups<ROWS>(c, s, M, ld, n, fl, p[k0], p[k1]);
