@@ -542,13 +542,12 @@ __device__ __forceinline__ unsigned warp_gj_panel(double *M, int ldm, int n, int
 #pragma unroll
     for (int c = 0; c < 8; ++c) a[t][c] = (r < n && c < ib) ? Mp[r + c * ldm] : 0.0;
   }
-  // one step on the register column K (the panel's column k)
-  const auto step = [&](int k, auto KC) {
-    constexpr int K = decltype(KC)::v;
+  // one step: the panel's column k, in the registers' column 0
+  const auto step = [&](int k) {
     unsigned key = 0;
 #pragma unroll
     for (int t = 0; t < T; ++t) {
-      const unsigned h = ((unsigned)__double2hiint(fabs(a[t][K])) & 0xFFFFFF00u) |
+      const unsigned h = ((unsigned)__double2hiint(fabs(a[t][0])) & 0xFFFFFF00u) |
                          (unsigned)(255 - (lane + 32 * t));
       if (!((used >> t) & 1u)) key = max(key, h);
     }
@@ -558,45 +557,34 @@ __device__ __forceinline__ unsigned warp_gj_panel(double *M, int ldm, int n, int
     pick_row<0, T>(ot, a, u);                       // uniform branches
 #pragma unroll
     for (int c = 0; c < 8; ++c) u[c] = __shfl_sync(Z2_FULL, u[c], ol);
-    const double rd = rcp_newton(u[K]);
+    const double rd = rcp_newton(u[0]);
     if (lane == 0) piv[j0 + k] = br;
 #pragma unroll
     for (int c = 0; c < 8; ++c) u[c] *= rd;
 #pragma unroll
     for (int t = 0; t < T; ++t) {
       const bool isp = t == ot && lane == ol;
-      const double l = isp ? 0.0 : a[t][K];
+      const double l = isp ? 0.0 : a[t][0];
 #pragma unroll
-      for (int c = 0; c < 8; ++c)
-        if (c != K) a[t][c] = fma(-l, u[c], a[t][c]);
-      a[t][K] = isp ? 1.0 : -l * rd;
+      for (int c = 1; c < 8; ++c) a[t][c] = fma(-l, u[c], a[t][c]);
+      a[t][0] = isp ? 1.0 : -l * rd;
       if (isp) { scl[t] = rd; used |= 1u << t; }
     }
   };
-  if constexpr (Z2_NT == 128) {
-    // a loop over the columns, the current one rotated to the front: 16 T moves
-    // a step for an eighth of the code, which pays where several blocks share
-    // an SM's instruction cache (alone at N = 64: 42 K cycles against 34 K)
+  // a loop over the columns, the current one rotated to the front: 8 T moves a
+  // step for an eighth of the code (unrolled, alone on an SM: the same within 1 %
+  // at N = 36 ... 144; the SM's instruction cache is shared by several blocks in
+  // the 128-thread build)
 #pragma unroll 1
-    for (int k = 0; k < 8; ++k) {
-      if (k < ib) step(k, WyIdx<0>{});
+  for (int k = 0; k < 8; ++k) {
+    if (k < ib) step(k);
 #pragma unroll
-      for (int t = 0; t < T; ++t) {
-        const double f = a[t][0];
+    for (int t = 0; t < T; ++t) {
+      const double f = a[t][0];
 #pragma unroll
-        for (int c = 0; c < 7; ++c) a[t][c] = a[t][c + 1];
-        a[t][7] = f;
-      }
+      for (int c = 0; c < 7; ++c) a[t][c] = a[t][c + 1];
+      a[t][7] = f;
     }
-  } else {
-    if (0 < ib) step(0, WyIdx<0>{});
-    if (1 < ib) step(1, WyIdx<1>{});
-    if (2 < ib) step(2, WyIdx<2>{});
-    if (3 < ib) step(3, WyIdx<3>{});
-    if (4 < ib) step(4, WyIdx<4>{});
-    if (5 < ib) step(5, WyIdx<5>{});
-    if (6 < ib) step(6, WyIdx<6>{});
-    if (7 < ib) step(7, WyIdx<7>{});
   }
   const int n8 = (n + 7) & ~7;
 #pragma unroll

@@ -2,8 +2,8 @@
 //
 // Each warp forms units of (8 RT) x (8 CT) entries over the whole k range,
 // straight from global or shared memory: an operand fragment is used for RT or
-// CT products, and the fragments of the next eight k values are in flight while
-// the current eight are multiplied.
+// CT products.  (Loading the next eight k values ahead of the products in the
+// middle units: 0.5 % slower bins at N = 64, 1 % at N = 100.)
 #pragma once
 #include "z2_blocked.cuh"
 
@@ -63,32 +63,11 @@ __device__ __forceinline__ void gemm_unit(int n, MatRef A, MatRef B, int r0, int
 #pragma unroll
       for (int b = 0; b < CT; ++b) dmma884(acc[a][b][0], acc[a][b][1], fa[a].y, fb[b].y);
   };
-  if constexpr (Z2_NT == 256 && RT * CT >= 8 && RT * CT <= 14) {
-    // middle units: the operands of the next eight k values are in flight behind
-    // the products (an L2 latency is several times their issue time; N = 64
-    // 15 -> 12 K cycles).  The largest have no registers left for it, the
-    // smallest too few k steps.
-    int l = lb + 2 * lc;
-    const int last = n8 - 8 + 2 * lc;
-    double2 fa[2][RT], fb[2][CT];
-    if (l <= last) load(fa[0], fb[0]);
 #pragma unroll 1
-    while (l <= last) {
-      if (l + 8 <= last) load(fa[1], fb[1]);
-      mul(l, fa[0], fb[0]);
-      l += 8;
-      if (l > last) break;
-      if (l + 8 <= last) load(fa[0], fb[0]);
-      mul(l, fa[1], fb[1]);
-      l += 8;
-    }
-  } else {
-#pragma unroll 1
-    for (int l = lb + 2 * lc; l < n8; l += 8) {
-      double2 fa[RT], fb[CT];
-      load(fa, fb);
-      mul(l, fa, fb);
-    }
+  for (int l = lb + 2 * lc; l < n8; l += 8) {
+    double2 fa[RT], fb[CT];
+    load(fa, fb);
+    mul(l, fa, fb);
   }
   if (n8 < n) {              // four trailing k values
     const int l = n8 + lc;
@@ -172,9 +151,9 @@ __device__ __forceinline__ void gemm_sized(int n, MatRef A, const int *rowmap, M
 // The product in units that cut the (N / 8)^2 tiles into a multiple of the four
 // sub-partitions' tensor pipes where they can (18 x 18 tiles: 12 units of 3 x 9,
 // three per sub-partition), with as many products per fragment as registers
-// allow: N = 144 takes 80 K cycles against 103 K for 16 x 16 groups (47 K at the
-// SM's DMMA rate; the fragment loads' trips to L2 are the rest).  a_upper: A(i, l) reads as 0 for i > l; b_lower: B(l, j) reads as 0 for
-// l < j.
+// allow: N = 144 takes 90 K cycles against 103 K for 16 x 16 groups (47 K at the
+// SM's DMMA rate; the fragment loads' trips to L2 are the rest).  a_upper: A(i, l)
+// reads as 0 for i > l; b_lower: B(l, j) reads as 0 for l < j.
 static __device__ __noinline__ void gemm_nnn(int n, MatRef A, const int *rowmap, bool a_upper, MatRef B,
                                       bool b_lower, GemmOut out) {
   const bool va = A.cs == 1 && (A.rs & 1) == 0 && ((uintptr_t)A.p & 15) == 0;
