@@ -21,7 +21,7 @@ OUT = os.path.join(HERE, "libz2dqmc.so")
 # once, and for this one that took over ten minutes; function by function it
 # takes half a minute.  The device functions are static, so that the compiler
 # still sees all their callers (address spaces, constants): with external linkage
-# the time-displaced correlators took a quarter longer.
+# the time-displaced correlators took up to 39 % longer.
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = [*ARCH, "-O3", "-lineinfo", "-std=c++17", "-dc", "-Xcompiler", "-fPIC"]
 

@@ -14,8 +14,7 @@
 // three sweeps over lines: a thread loads one line (or two neighbouring ones)
 // of a matrix column (or of two neighbouring matrix rows) into registers as
 // 16-byte words, applies its passes (E3 E3 as one rotation) and stores it, so
-// the matrix crosses shared memory three times per product.  A warp keeps a
-// line's coefficients in registers while it works through the matrix.
+// the matrix crosses shared memory three times per product.
 //
 // Bound: shared-memory bandwidth.  N = 144: the two products of a slice move
 // 2 MB, 15.5 K cycles at 128 B/clk; the previous sweeps (generic addresses,

@@ -37,9 +37,9 @@ __device__ __forceinline__ unsigned int ranf_pow(int n) {
 // Bound: the latency of the round (the ratio, two barriers, the loop over the
 // queued columns), not the arithmetic.  Evaluating from X and Yt for 32
 // proposals at a time in one warp, as this did before, cost a loop over the
-// queued columns per batch and a batch per 32 rejections: 3.8 to 5.7 K cycles
-// per accept, now 1957 (L = 4), 1738 (8), 2728 (10), 2891 (12), one chain
-// alone on its SM.  Keeping G in the
+// queued columns per batch and a batch per 32 rejections: 3.8 K cycles per accept
+// at L = 8 and, in two measurements, 5.7 and 6.6 K at L = 12; now 1957 (L = 4), 1738
+// (8), 2728 (10), 2891 (12), one chain alone on its SM.  Keeping G in the
 // register file instead (an update per accept, no queue) lost the gain to
 // picking the accepted rows and columns out of the registers.
 // GS: G is in shared memory.

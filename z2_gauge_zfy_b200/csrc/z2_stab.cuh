@@ -139,7 +139,7 @@ static __device__ __noinline__ void dev_stab_green(const Smem &s, int N, int nt,
 // column order of D may differ).
 //
 // Every step is a panel kernel of z2_blocked.cuh or a product of z2_gemm.cuh.
-// At N = 144 (cycles, one SM): QR 188 K, Q 93 K, inverse 154 K, a product 83 K;
+// At N = 144 (cycles, one SM): QR 175 K, Q 95 K, inverse 170 K, a product 90 K;
 // the register-resident kernels they replace (one column per step over the
 // whole tile) took 393 K, 188 K, 298 K and 103 K.
 // ---------------------------------------------------------------------------
